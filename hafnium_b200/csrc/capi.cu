@@ -14,6 +14,7 @@
 
 #include "../../include/hfjk.h"
 #include "context.cuh"
+#include "coulomb.cuh"
 #include "dgemm.cuh"
 #include "integrals.cuh"
 #include "jk.cuh"
@@ -89,6 +90,7 @@ struct hf_ctx {
     size_t ctc_bytes = 0;
     int* d_info = nullptr;
     double* d_scalar = nullptr;
+    int* h_flag = nullptr;  // page-locked error flag of kernels whose waits are bounded (flag_slot), or null
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // rows [row0, row1) of the fitted tensor held here (internal auxiliary order;
     // row1 < 0: all of them), for a tensor sharded over devices by auxiliary index
@@ -208,6 +210,39 @@ const double* shared_boys_table(int device) {
         tables[device] = p;
     }
     return tables[device];
+}
+
+// Page-locked error flags, one per live context: a kernel with bounded waits
+// writes its flag only when a wait runs out, so the host reads it after the
+// stream's synchronisation without a copy. One page for the process, kept until
+// it exits; a context that finds no free slot gets null and its builds use the
+// kernels that wait for nothing.
+constexpr int kFlagSlots = 1024;
+std::mutex g_flag_mutex;
+int* g_flag_page = nullptr;
+std::vector<int> g_flag_free;
+
+int* flag_slot() {
+    std::lock_guard<std::mutex> lock(g_flag_mutex);
+    if (!g_flag_page) {
+        if (cudaHostAlloc((void**)&g_flag_page, sizeof(int) * kFlagSlots, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            g_flag_page = nullptr;
+            return nullptr;
+        }
+        for (int i = kFlagSlots - 1; i >= 0; --i) g_flag_free.push_back(i);
+    }
+    if (g_flag_free.empty()) return nullptr;
+    int* p = g_flag_page + g_flag_free.back();
+    g_flag_free.pop_back();
+    *p = 0;
+    return p;
+}
+
+void flag_release(int* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(g_flag_mutex);
+    g_flag_free.push_back((int)(p - g_flag_page));
 }
 
 // Retained device blocks: the fitted tensor and its BF16 copy (tens of GB at the
@@ -628,6 +663,7 @@ int hf_ctx_create(int device, hf_ctx** out) {
     upload_c2s(ctx->stream);
     keep_pool_memory(device);
     ctx->d_btable = shared_boys_table(device);
+    ctx->h_flag = flag_slot();
     if (!ctx->d_btable || alloc(ctx, (void**)&ctx->d_info, 4 * sizeof(int)) != HF_OK ||
         alloc(ctx, (void**)&ctx->d_scalar, 4 * sizeof(double)) != HF_OK) {
         hf_ctx_destroy(ctx);
@@ -666,6 +702,7 @@ int hf_ctx_destroy(hf_ctx* ctx) {
     schedule_release(ctx);
     release(ctx, ctx->d_info);
     release(ctx, ctx->d_scalar);
+    flag_release(ctx->h_flag);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->own) cudaStreamDestroy(ctx->own);
@@ -1117,6 +1154,36 @@ static JkPlan plan_of(const hf_ctx* ctx) {
     return p;
 }
 
+// The one-pass J build where it applies, else the two-pass one; returns once J is
+// complete. work holds coulomb_doubles(ctx, p).
+static size_t coulomb_doubles(const hf_ctx* ctx, const JkPlan& p, bool* fused) {
+    const size_t need = ctx->h_flag ? coulomb_fused_work_doubles(p) : 0;
+    *fused = need > 0;
+    return need ? need : (size_t)coulomb_work_doubles(p);
+}
+
+static int coulomb_run(hf_ctx* ctx, const JkPlan& p, bool fused, const double* D, double* J, double* work,
+                       double* host_out, const char* what) {
+    const size_t bytes = sizeof(double) * (size_t)p.n * p.n;
+    if (!fused) {
+        HF_CU(coulomb_build(p, D, J, work, ctx->stream));
+        ctx->stats.kernel_launches += 4;
+        if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        return check_async(ctx, what);
+    }
+    std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
+    if (coulomb_fused_cooperative(p)) lock.lock();
+    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, ctx->h_flag, ctx->wait_ns, ctx->stream));
+    ++ctx->stats.kernel_launches;
+    if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    const int s = check_async(ctx, what);
+    if (s == HF_OK && *(volatile int*)ctx->h_flag != 0) {
+        *(volatile int*)ctx->h_flag = 0;
+        return fail(ctx, HF_ERR_TIMEOUT, std::string(what) + ": a wait between the kernel's CTAs ran out");
+    }
+    return s;
+}
+
 int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
     if (!ctx || !D || !J) return HF_ERR_ARG;
     if (!ctx->built) return fail(ctx, HF_ERR_STATE, "build the fitted tensor first");
@@ -1124,7 +1191,9 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
     const JkPlan p = plan_of(ctx);
     const size_t nn = (size_t)ctx->n * ctx->n;
     int s;
-    if ((s = ensure_work(ctx, sizeof(double) * coulomb_work_doubles(p))) != HF_OK) return s;
+    bool fused = false;
+    const size_t need = coulomb_doubles(ctx, p, &fused);
+    if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
     const double* dD = D;
     double* dJ = J;
     if (!on_device) {
@@ -1134,11 +1203,9 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
         dJ = ctx->d_io + nn;
     }
     time_begin(ctx);
-    HF_CU(coulomb_build(p, dD, dJ, ctx->d_work, ctx->stream));
-    ctx->stats.kernel_launches += 4;
-    if (!on_device) HF_CU(cudaMemcpyAsync(J, dJ, nn * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    s = coulomb_run(ctx, p, fused, dD, dJ, ctx->d_work, on_device ? nullptr : J, "hf_coulomb");
     ctx->stats.ms_coulomb = time_end(ctx);
-    return check_async(ctx, "hf_coulomb");
+    return s;
 }
 
 // K from Ct ([opad][npad], device) and sign ([opad]).
@@ -2134,9 +2201,8 @@ extern "C" int hf_coulomb_static(hf_ctx* ctx, const double* density, double* cou
     int s = static_scratch(ctx, &scratch);
     if (s != HF_OK) return s;
     const JkPlan p = plan_of(ctx);
-    if (coulomb_work_doubles(p) > kStaticScratchDoubles) return fail(ctx, HF_ERR_ARG, "scratch size exceeded");
-    cudaError_t e = coulomb_build(p, density, coulomb, scratch, ctx->stream);
-    if (e != cudaSuccess) return fail(ctx, HF_ERR_CUDA, std::string("hf_coulomb_static: ") + cudaGetErrorString(e));
-    ctx->stats.kernel_launches += 4;
-    return check_async(ctx, "hf_coulomb_static");
+    bool fused = false;
+    if (coulomb_doubles(ctx, p, &fused) > (size_t)kStaticScratchDoubles)
+        return fail(ctx, HF_ERR_ARG, "scratch size exceeded");
+    return coulomb_run(ctx, p, fused, density, coulomb, scratch, nullptr, "hf_coulomb_static");
 }

@@ -1,0 +1,54 @@
+"""The one-pass Coulomb build against a plain contraction of the fitted tensor it reads (B200)."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from hafnium_b200.basis import ShellTable
+from hafnium_b200.jk import B200DensityFittedCoulombExchange
+
+pytestmark = pytest.mark.gpu
+
+
+def hydrogens(n, n_aux):
+    """A builder with exactly n orbital and n_aux auxiliary functions: s shells on a jittered grid."""
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(max(n, n_aux) ** (1 / 3)))
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    at = 1.4 * grid + rng.uniform(-0.2, 0.2, size=grid.shape)
+    return B200DensityFittedCoulombExchange.from_tables(ShellTable.build("sto-3g", ["H"] * n, at[:n]),
+                                                        ShellTable.build("sto-3g", ["H"] * n_aux, at[:n_aux]))
+
+
+# one piece, odd counts, the tile edges, each form of the exchange between CTAs (none, by lanes, by
+# warps, through owners), each pieces-per-thread variant, and sizes past the one-pass form's range
+@pytest.mark.parametrize("n,n_aux", [(1, 1), (2, 3), (7, 5), (24, 113), (63, 17), (64, 200), (65, 31), (127, 260),
+                                     (129, 300), (193, 64), (257, 129), (390, 150), (520, 131), (777, 70), (1030, 67),
+                                     (1410, 40), (1537, 33), (1601, 20)])
+def test_coulomb_of_every_layout(n, n_aux):
+    import torch
+
+    two_body = hydrogens(n, n_aux)
+    gen = torch.Generator().manual_seed(n)
+    d = torch.randn((n, n), dtype=torch.float64, generator=gen).cuda()
+    d = d + d.T
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = two_body.orbital_tensor(eye, eye)
+    terms = torch.einsum("quv,uv->q", b, d)
+    expected = torch.einsum("quv,q->uv", b, terms)
+    # two sums of n^2 and n_aux rounded products in another order: each errs by at most its
+    # length times eps times the sum of its absolute terms
+    size = torch.einsum("quv,q->uv", b.abs(), torch.einsum("quv,uv->q", b.abs(), d.abs()))
+    bound = (2.3e-16 * (n * n + n_aux) * size).clamp(min=1e-300)
+    for _ in range(2):
+        got = two_body.coulomb(d)
+        assert float(((got - expected).abs() / bound).max()) < 1.0
+        assert float((got - got.T).abs().max()) == 0.0
+    again = two_body.coulomb(d)
+    if n <= 1030:
+        assert torch.equal(again, got)  # sums in a fixed order
+    # J may overwrite D
+    inplace = d.clone()
+    two_body.context.coulomb_device(inplace, inplace)
+    assert float(((inplace - expected).abs() / bound).max()) < 1.0
