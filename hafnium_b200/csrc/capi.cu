@@ -1193,7 +1193,11 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
     int s;
     bool fused = false;
     const size_t need = coulomb_doubles(ctx, p, &fused);
-    if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
+    if (ctx->work_bytes < sizeof(double) * need) {
+        if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
+        // the one-pass build tells its packets from what the block held before by their tags
+        HF_CU(cudaMemsetAsync(ctx->d_work, 0, ctx->work_bytes, ctx->stream));
+    }
     const double* dD = D;
     double* dJ = J;
     if (!on_device) {

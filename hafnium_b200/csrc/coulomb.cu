@@ -727,7 +727,20 @@ size_t packet_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql
 size_t sum_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b; }
 size_t jpart_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ge * a.pp; }
 
-std::atomic<uint32_t> g_tag{1};
+// Tags count up within [kTagBase, kTagBase + kTagCount): as integers, floats or halves of doubles
+// these words do not occur in the data that other kernels leave in the same memory (small counts
+// did), and a tag comes back only after 2^28 row blocks.
+constexpr uint32_t kTagBase = 0x80000000u, kTagCount = 1u << 28;
+std::atomic<uint32_t> g_tag{0};
+
+// The first of `count` consecutive tags.
+uint32_t take_tags(uint32_t count) {
+    uint32_t at = g_tag.load(), from;
+    do {
+        from = at + count <= kTagCount ? at : 0;
+    } while (!g_tag.compare_exchange_weak(at, from + count));
+    return kTagBase + from;
+}
 
 int device_sms() {
     static std::atomic<int> sms[64];
@@ -777,7 +790,7 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     a.jpart = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(a.sums) + sum_bytes(a));
     a.jflag = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(a.jpart) + jpart_bytes(a));
     a.stop = reinterpret_cast<uint32_t*>(a.jflag + (size_t)a.gq * a.ge);
-    a.tag = g_tag.fetch_add((uint32_t)a.blocks + 1);
+    a.tag = take_tags((uint32_t)a.blocks + 1);
     a.err = err;
     a.wait_ns = wait_ns;
     switch (f.ept) {

@@ -11,7 +11,8 @@ namespace hf {
 
 // The Coulomb build of one cluster in one pass over B (coulomb.cu). Applies when
 // coulomb_fused_work_doubles(p) > 0 (the slices of J and D fit the registers of
-// one CTA per SM: n up to about 1100); work holds that many doubles.
+// one CTA per SM: n up to about 1100); work holds that many doubles, zeroed once
+// when it is allocated.
 size_t coulomb_fused_work_doubles(const JkPlan& p);
 
 // J = scale * sum_q (B_q . D) B_q, J full n x n. The grid's CTAs wait on one another,

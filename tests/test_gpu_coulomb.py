@@ -52,3 +52,26 @@ def test_coulomb_of_every_layout(n, n_aux):
     inplace = d.clone()
     two_body.context.coulomb_device(inplace, inplace)
     assert float(((inplace - expected).abs() / bound).max()) < 1.0
+
+
+def test_the_first_coulomb_builds_of_a_process():
+    """The packets between CTAs are told by their tags from what the memory held before: a fresh process,
+    whose tags start anew in memory that the build's integer lists have just used."""
+    import subprocess
+    import sys
+
+    code = """
+import numpy as np, torch
+from hafnium_b200.jk import B200DensityFittedCoulombExchange
+from tests.helpers import molecule, tables
+for tag in ("water", "h2o2_s0", "h2o4_s1"):
+    orb, aux = tables(molecule(tag))
+    for rep in range(2):
+        two_body = B200DensityFittedCoulombExchange.from_tables(orb, aux)
+        n = two_body.n_ao
+        d = torch.randn((n, n), dtype=torch.float64, device="cuda")
+        d = d + d.T
+        first, second = two_body.coulomb(d), two_body.coulomb(d)
+        assert torch.equal(first, second), (tag, rep, float((first - second).abs().max()))
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
