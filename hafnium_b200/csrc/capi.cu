@@ -245,6 +245,53 @@ void flag_release(int* p) {
     g_flag_free.push_back((int)(p - g_flag_page));
 }
 
+// Side streams for Branches: one set per device, kept until the process exits and
+// lent to one call at a time; a call that finds it lent launches on its own stream
+// alone. (Several contexts built at once, as by the batched SCF's host threads,
+// already run beside one another; a set for each took 64 instead of 38 ms for
+// twelve clusters, in the driver's stream and event calls.)
+std::mutex g_branch_mutex;
+Branches g_branches[64];
+bool g_branches_lent[64] = {};
+
+struct BranchLoan {
+    hf_ctx* ctx;
+    Branches br;
+    explicit BranchLoan(hf_ctx* c) : ctx(c) {
+        br.main = c->stream;
+        if (c->device < 0 || c->device >= 64) return;
+        std::lock_guard<std::mutex> lock(g_branch_mutex);
+        Branches& set = g_branches[c->device];
+        if (g_branches_lent[c->device]) return;
+        if (!set.have) {
+            bool ok = true;
+            for (auto& q : set.side) ok = ok && cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) == cudaSuccess;
+            for (auto& q : set.event) ok = ok && cudaEventCreateWithFlags(&q, cudaEventDisableTiming) == cudaSuccess;
+            if (!ok) {
+                cudaGetLastError();
+                for (auto& q : set.side)
+                    if (q) cudaStreamDestroy(q);
+                for (auto& q : set.event)
+                    if (q) cudaEventDestroy(q);
+                set = Branches{};
+                return;
+            }
+            set.have = true;
+        }
+        g_branches_lent[c->device] = true;
+        br = set;
+        br.main = c->stream;
+    }
+    ~BranchLoan() {
+        if (!br.have) return;
+        br.join();  // also on an error path: the context's stream ends after what was forked
+        std::lock_guard<std::mutex> lock(g_branch_mutex);
+        g_branches_lent[ctx->device] = false;
+    }
+    BranchLoan(const BranchLoan&) = delete;
+    BranchLoan& operator=(const BranchLoan&) = delete;
+};
+
 // Retained device blocks: the fitted tensor and its BF16 copy (tens of GB at the
 // largest clusters) and the J/K scratch areas. A context that is destroyed, or
 // that rebuilds for another molecule, hands its blocks of at least
@@ -872,8 +919,13 @@ int hf_dims(const hf_ctx* ctx, int64_t* n_ao, int64_t* n_aux) {
 static int build_metric(hf_ctx* ctx) {
     const size_t bytes = sizeof(double) * (size_t)ctx->naux * ctx->naux;
     if (!ctx->d_metric && alloc(ctx, (void**)&ctx->d_metric, bytes)) return HF_ERR_OOM;
-    HF_CU(launch_metric(ctx->d_aux, ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable,
-                        ctx->d_metric, ctx->naux, ctx->stream));
+    {
+        BranchLoan loan(ctx);
+        HF_CU(loan.br.fork());
+        HF_CU(launch_metric(ctx->d_aux, ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable,
+                            ctx->d_metric, ctx->naux, loan.br));
+        HF_CU(loan.br.join());
+    }
     ctx->stats.kernel_launches += 25;
     return check_async(ctx, "metric");
 }
@@ -957,20 +1009,42 @@ static int three_center_chunk(hf_ctx* ctx, int row0, int row1, double* T, PairTa
     int max_npp[3][3];
     chunk_tasks(ctx, row0, row1, tasks, max_npp);
     ChunkDesc cd{row0, row1, ctx->nt, tile_index(row0, row0, ctx->nt), ctx->naux};
-    size_t off = 0;
+    size_t off = 0, most = 0, pairs = 0;
+    for (int la = 0; la <= 2; ++la)
+        for (int lb = la; lb <= 2; ++lb) {
+            pairs += tasks[la][lb].size();
+            most = std::max(most, tasks[la][lb].size() * (size_t)pair_data_stride(la, lb, max_npp[la][lb]));
+        }
+    if (pairs > task_cap) return fail(ctx, HF_ERR_STATE, "task buffer too small");
+    double* data = nullptr;
+    int* npps = nullptr;
+    if (talloc(ctx, (void**)&data, sizeof(double) * most) || talloc(ctx, (void**)&npps, sizeof(int) * (pairs + 1))) {
+        trelease(ctx, data);
+        return HF_ERR_OOM;
+    }
+    Branches one;  // no side streams
+    one.main = ctx->stream;
+    cudaError_t e = cudaSuccess;
     for (int la = 0; la <= 2; ++la)
         for (int lb = la; lb <= 2; ++lb) {
             auto& v = tasks[la][lb];
-            if (v.empty()) continue;
-            if (off + v.size() > task_cap) return fail(ctx, HF_ERR_STATE, "task buffer too small");
-            HF_CU(cudaMemcpyAsync(d_tasks + off, v.data(), sizeof(PairTask) * v.size(), cudaMemcpyHostToDevice,
-                                  ctx->stream));
-            HF_CU(launch_three_center(la, lb, d_tasks + off, (int)v.size(), max_npp[la][lb], ctx->d_orb, ctx->d_aux,
-                                      ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable, cd,
-                                      T, ctx->stream));
-            ctx->stats.kernel_launches += 5;
+            if (v.empty() || e != cudaSuccess) continue;
+            const PairData pd{data, pair_data_stride(la, lb, max_npp[la][lb]), npps + off};
+            e = cudaMemcpyAsync(d_tasks + off, v.data(), sizeof(PairTask) * v.size(), cudaMemcpyHostToDevice,
+                                ctx->stream);
+            if (e == cudaSuccess)
+                e = launch_pair_data(la, lb, d_tasks + off, (int)v.size(), max_npp[la][lb], ctx->d_orb, ctx->d_exps,
+                                     ctx->d_coefs, pd, ctx->stream);
+            if (e == cudaSuccess)
+                e = launch_three_center(la, lb, d_tasks + off, (int)v.size(), max_npp[la][lb], ctx->d_orb, ctx->d_aux,
+                                        ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable, cd,
+                                        pd, T, one);
+            ctx->stats.kernel_launches += 6;
             off += v.size();
         }
+    trelease(ctx, data);
+    trelease(ctx, npps);
+    HF_CU(e);
     // the host task vectors must outlive the async copies
     HF_CU(cudaStreamSynchronize(ctx->stream));
     return HF_OK;
@@ -1082,15 +1156,33 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
                 all_tasks.insert(all_tasks.end(), v.begin(), v.end());
             }
     }
-    double* T = nullptr;
+    // one chunk's pair data: every class of the largest chunk side by side
+    std::vector<size_t> data_at(6 * chunks.size() + 1, 0);
+    size_t data_doubles = 0;
+    for (size_t c = 0; c < chunks.size(); ++c) {
+        size_t at = 0;
+        for (size_t i = 0; i < launches[c].size(); ++i) {
+            const Launch& l = launches[c][i];
+            data_at[6 * c + i] = at;
+            at += l.count * (size_t)pair_data_stride(l.la, l.lb, l.max_npp);
+        }
+        data_doubles = std::max(data_doubles, at);
+    }
+    double *T = nullptr, *pair_data = nullptr;
     PairTask* d_tasks = nullptr;
+    int* d_npps = nullptr;
     if (talloc(ctx, (void**)&d_tasks, sizeof(PairTask) * std::max<size_t>(1, all_tasks.size())) ||
-        talloc(ctx, (void**)&T, budget)) {
+        talloc(ctx, (void**)&d_npps, sizeof(int) * std::max<size_t>(1, all_tasks.size())) ||
+        talloc(ctx, (void**)&pair_data, sizeof(double) * data_doubles) || talloc(ctx, (void**)&T, budget)) {
         trelease(ctx, T);
+        trelease(ctx, pair_data);
+        trelease(ctx, d_npps);
         trelease(ctx, d_tasks);
         trelease(ctx, Linv);
         return HF_ERR_OOM;
     }
+    BranchLoan loan(ctx);
+    Branches& br = loan.br;
     if (!all_tasks.empty())
         HF_CU(cudaMemcpyAsync(d_tasks, all_tasks.data(), sizeof(PairTask) * all_tasks.size(), cudaMemcpyHostToDevice,
                               ctx->stream));
@@ -1106,13 +1198,28 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
         cudaEventRecord(ev[3 * c], ctx->stream);
         e = cudaMemsetAsync(T, 0, sizeof(double) * (size_t)ncols * N, ctx->stream);
         const ChunkDesc cd{row0, row1, ctx->nt, t0, ctx->naux};
-        for (const Launch& l : launches[c]) {
-            if (e != cudaSuccess) break;
+        auto data_of = [&](size_t i) {
+            const Launch& l = launches[c][i];
+            return PairData{pair_data + data_at[6 * c + i], pair_data_stride(l.la, l.lb, l.max_npp), d_npps + l.off};
+        };
+        // the classes are independent of one another: first every pair's data, then every class
+        if (e == cudaSuccess) e = br.fork();
+        for (size_t i = 0; i < launches[c].size() && e == cudaSuccess; ++i) {
+            const Launch& l = launches[c][i];
+            e = launch_pair_data(l.la, l.lb, d_tasks + l.off, (int)l.count, l.max_npp, ctx->d_orb, ctx->d_exps,
+                                 ctx->d_coefs, data_of(i), br.next());
+            ++ctx->stats.kernel_launches;
+        }
+        if (e == cudaSuccess) e = br.join();
+        if (e == cudaSuccess) e = br.fork();
+        for (size_t i = 0; i < launches[c].size() && e == cudaSuccess; ++i) {
+            const Launch& l = launches[c][i];
             e = launch_three_center(l.la, l.lb, d_tasks + l.off, (int)l.count, l.max_npp, ctx->d_orb, ctx->d_aux,
-                                    ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable, cd, T,
-                                    ctx->stream);
+                                    ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable, cd,
+                                    data_of(i), T, br);
             ctx->stats.kernel_launches += 5;
         }
+        if (e == cudaSuccess) e = br.join();
         cudaEventRecord(ev[3 * c + 1], ctx->stream);
         if (e == cudaSuccess)
             e = apply_inverse_factor(Linv, N, N, T, N, ncols, ctx->d_B + t0 * 4096, ldb, ctx->stream, q_begin, q_end);
@@ -1133,6 +1240,8 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
         }
     for (auto& x : ev) cudaEventDestroy(x);
     trelease(ctx, T);
+    trelease(ctx, pair_data);
+    trelease(ctx, d_npps);
     trelease(ctx, d_tasks);
     trelease(ctx, Linv);
     if (e != cudaSuccess) return fail(ctx, HF_ERR_CUDA, std::string("fitted tensor: ") + cudaGetErrorString(e));
@@ -1672,9 +1781,12 @@ int hf_one_electron(hf_ctx* ctx, int kind, const double* charges, const double* 
     const size_t nn = (size_t)n * n;
     double* buf = nullptr;
     const int ns = (int)ctx->orb.size();
-    std::vector<int2> tasks[3][3];
+    std::vector<int2> tasks[3][3], all;
     for (int a = 0; a < ns; ++a)
         for (int b = 0; b < ns; ++b) tasks[ctx->orb[a].l][ctx->orb[b].l].push_back(make_int2(a, b));
+    all.reserve((size_t)ns * ns);
+    for (auto& r : tasks)
+        for (auto& v : r) all.insert(all.end(), v.begin(), v.end());
     const size_t need = sizeof(double) * (nn + 4 * (size_t)std::max<int64_t>(natoms, 1)) + sizeof(int2) * ns * ns + 64;
     if (talloc(ctx, (void**)&buf, need)) return HF_ERR_OOM;
     double* sOut = buf;
@@ -1689,17 +1801,23 @@ int hf_one_electron(hf_ctx* ctx, int kind, const double* charges, const double* 
     }
     double* dOut = on_device ? out : sOut;
     size_t off = 0;
-    cudaError_t e = cudaSuccess;
-    for (int la = 0; la <= 2 && e == cudaSuccess; ++la)
-        for (int lb = 0; lb <= 2 && e == cudaSuccess; ++lb) {
-            auto& v = tasks[la][lb];
-            if (v.empty()) continue;
-            cudaMemcpyAsync(dt + off, v.data(), sizeof(int2) * v.size(), cudaMemcpyHostToDevice, ctx->stream);
-            e = launch_one_electron(kind, la, lb, dt + off, (int)v.size(), ctx->d_orb, ctx->d_exps, ctx->d_coefs, sq,
-                                    spos, (int)natoms, ctx->d_btable, dOut, n, ctx->stream);
-            ++ctx->stats.kernel_launches;
-            off += v.size();
-        }
+    cudaError_t e = cudaMemcpyAsync(dt, all.data(), sizeof(int2) * all.size(), cudaMemcpyHostToDevice, ctx->stream);
+    {
+        BranchLoan loan(ctx);
+        Branches& br = loan.br;
+        if (e == cudaSuccess) e = br.fork();
+        for (int la = 0; la <= 2 && e == cudaSuccess; ++la)
+            for (int lb = 0; lb <= 2 && e == cudaSuccess; ++lb) {
+                auto& v = tasks[la][lb];
+                if (v.empty()) continue;
+                e = launch_one_electron(kind, la, lb, dt + off, (int)v.size(), ctx->d_orb, ctx->d_exps, ctx->d_coefs,
+                                        sq, spos, (int)natoms, ctx->d_btable, dOut, n, br.next());
+                ++ctx->stats.kernel_launches;
+                off += v.size();
+            }
+        const cudaError_t je = br.join();
+        if (e == cudaSuccess) e = je;
+    }
     if (e == cudaSuccess && !on_device)
         e = cudaMemcpyAsync(out, sOut, sizeof(double) * nn, cudaMemcpyDeviceToHost, ctx->stream);
     trelease(ctx, buf);
@@ -1947,8 +2065,12 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
     HF_CU(gemm((int)N, (int)N, (int)oo, G, oo, G, oo, WK, N, 1.0, 0, 3));  // upper tiles only
     ctx->stats.ms_gradient_weights += time_end(ctx);
     time_begin(ctx);
+    BranchLoan loan(ctx);  // the force sums are atomic: the classes may run beside one another
+    Branches& br = loan.br;
+    HF_CU(br.fork());
     HF_CU(launch_metric_grad(ctx->d_aux, ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable,
-                             WJ, WK, N, gaux, ctx->stream));
+                             WJ, WK, N, gaux, br));
+    HF_CU(br.join());
     ctx->stats.kernel_launches += 25;
     ctx->stats.ms_gradient_metric = time_end(ctx);
     time_begin(ctx);
@@ -1985,21 +2107,25 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
         return fail(ctx, HF_ERR_OOM, "no room for the gradient's pair list and pair data");
     HF_CU(cudaMemcpyAsync(d_pair_off, pair_off.data(), sizeof(int64_t) * (ntask + 1), cudaMemcpyHostToDevice,
                           ctx->stream));
+    std::vector<PairTask> all_tasks;
+    for (int la = 0; la <= 2; ++la)
+        for (int lb = la; lb <= 2; ++lb) all_tasks.insert(all_tasks.end(), tasks[la][lb].begin(), tasks[la][lb].end());
+    HF_CU(cudaMemcpyAsync(d_tasks, all_tasks.data(), sizeof(PairTask) * ntask, cudaMemcpyHostToDevice, ctx->stream));
+    HF_CU(br.fork());
     {
         size_t off = 0;
         for (int la = 0; la <= 2; ++la)
             for (int lb = la; lb <= 2; ++lb) {
                 auto& v = tasks[la][lb];
                 if (v.empty()) continue;
-                HF_CU(cudaMemcpyAsync(d_tasks + off, v.data(), sizeof(PairTask) * v.size(), cudaMemcpyHostToDevice,
-                                      ctx->stream));
                 HF_CU(launch_grad_pair_data(la, lb, d_tasks + off, (int)v.size(), max_npp[la][lb], ctx->d_orb,
                                             ctx->d_exps, ctx->d_coefs, Dt, n,
-                                            GradPairData{d_pair_off + off, pair_data, d_npps + off}, ctx->stream));
+                                            GradPairData{d_pair_off + off, pair_data, d_npps + off}, br.next()));
                 ++ctx->stats.kernel_launches;
                 off += v.size();
             }
     }
+    HF_CU(br.join());
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
     const size_t per_p = sizeof(double) * (nn + (size_t)n * o);
@@ -2029,6 +2155,7 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
             count[l] = std::max(0, hi - lo);
         }
         const GradWeights gw{Dt, cfit, GK, n, P0, Pb};
+        HF_CU(br.fork());
         size_t off = 0;
         for (int la = 0; la <= 2; ++la)
             for (int lb = la; lb <= 2; ++lb) {
@@ -2037,10 +2164,11 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
                 HF_CU(launch_three_center_grad(la, lb, d_tasks + off, (int)v.size(), max_npp[la][lb], ctx->d_orb,
                                                ctx->d_aux, ctx->d_exps, ctx->d_coefs, alist, count, ctx->d_btable, gw,
                                                GradPairData{d_pair_off + off, pair_data, d_npps + off}, gorb, gaux,
-                                               ctx->stream));
+                                               br));
                 ctx->stats.kernel_launches += 5;
                 off += v.size();
             }
+        HF_CU(br.join());  // the next block overwrites GK
         s0 = s1;
     }
     ctx->stats.ms_gradient_three_center = time_end(ctx);
@@ -2051,21 +2179,26 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
         for (int b = 0; b < nso; ++b) pairs1[ctx->orb[a].l][ctx->orb[b].l].push_back(make_int2(a, b));
     int2* d_pairs1 = reinterpret_cast<int2*>(tmp.take(((size_t)nso * nso * sizeof(int2) + 7) / 8 + 1));
     if (!d_pairs1) return fail(ctx, HF_ERR_OOM, "no room for the one-electron pair list");
+    std::vector<int2> all1;
+    all1.reserve((size_t)nso * nso);
+    for (auto& r : pairs1)
+        for (auto& v : r) all1.insert(all1.end(), v.begin(), v.end());
+    HF_CU(cudaMemcpyAsync(d_pairs1, all1.data(), sizeof(int2) * all1.size(), cudaMemcpyHostToDevice, ctx->stream));
+    HF_CU(br.fork());
     {
         size_t off = 0;
         for (int la = 0; la <= 2; ++la)
             for (int lb = 0; lb <= 2; ++lb) {
                 auto& v = pairs1[la][lb];
                 if (v.empty()) continue;
-                HF_CU(cudaMemcpyAsync(d_pairs1 + off, v.data(), sizeof(int2) * v.size(), cudaMemcpyHostToDevice,
-                                      ctx->stream));
                 HF_CU(launch_one_electron_grad(la, lb, d_pairs1 + off, (int)v.size(), ctx->d_orb, ctx->d_exps,
                                                ctx->d_coefs, dq, dpos, (int)natoms, ctx->d_btable, Dt, dW, n, gorb1,
-                                               gatom, ctx->stream));
+                                               gatom, br));
                 ctx->stats.kernel_launches += 2;
                 off += v.size();
             }
     }
+    HF_CU(br.join());
     ctx->stats.ms_gradient_one_electron = time_end(ctx);
     std::vector<double> h((size_t)(2 * nso + nsa) * 6 + 3 * natoms);
     HF_CU(cudaMemcpyAsync(h.data(), acc, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));

@@ -34,8 +34,9 @@ struct GradPairLayout {
     static constexpr int NSA = nsph(LA), NSB = nsph(LB), NSAB = NSA * NSB;
     static constexpr int KA = kMaxOrbContr[LA], KB = kMaxOrbContr[LB], KK = KA * KB;
     static constexpr int NH = ntet(LA + LB), NH1 = ntet(LA + LB + 1);
-    // per primitive pair: p, Px, Py, Pz | cc[KK] | E[NSAB][NH] | EA[3][NSAB][NH1] | EJ[NH] | EJA[3][NH1]
-    static constexpr int OFF_E = 4 + KK;
+    // per primitive pair: p, Px, Py, Pz, 1/p | cc[KK] | E[NSAB][NH] | EA[3][NSAB][NH1] | EJ[NH] | EJA[3][NH1]
+    static constexpr int INV = 4, CC = 5;
+    static constexpr int OFF_E = CC + KK;
     static constexpr int OFF_EA = OFF_E + NSAB * NH;
     static constexpr int OFF_EJ = OFF_EA + 3 * NSAB * NH1;
     static constexpr int OFF_EJA = OFF_EJ + NH;
@@ -51,6 +52,7 @@ __device__ int grad_pair_prologue(const DevShell& A, const DevShell& B, const do
                                   double* smem, int* s_pos) {
     using PL = GradPairLayout<LA, LB>;
     constexpr int NCA = ncart(LA), NCB = ncart(LB);
+    int* s_src = s_pos + kMaxPrimPairs + 1;  // the surviving primitive pairs, in order
     const int npp = A.nprim * B.nprim;
     const double abx = A.x - B.x, aby = A.y - B.y, abz = A.z - B.z;
     const double rab2 = abx * abx + aby * aby + abz * abz;
@@ -68,127 +70,101 @@ __device__ int grad_pair_prologue(const DevShell& A, const DevShell& B, const do
         int k = 0;
         for (int pp0 = 0; pp0 < npp; ++pp0) {
             const int keep = s_pos[pp0];
-            s_pos[pp0] = keep ? k : -1;
+            if (keep) s_src[k] = pp0;
             k += keep;
         }
         s_pos[kMaxPrimPairs] = k;
     }
     __syncthreads();
-    for (int pp0 = threadIdx.x; pp0 < npp; pp0 += blockDim.x) {
-        const int pp = s_pos[pp0];
-        if (pp < 0) continue;
+    // One task per (surviving primitive pair, spherical component pair, row): row 0 is the pair's
+    // values E[m], rows 1..3 the derivatives EA[d][m]; each task builds that pair's one-axis tables
+    // itself. A thread per primitive pair left one thread with all 100 rows of a d-d pair (1.2 ms).
+    const int nk = s_pos[kMaxPrimPairs];
+    for (int w = threadIdx.x; w < nk * PL::NSAB * 4; w += blockDim.x) {
+        const int pp = w / (PL::NSAB * 4), rest = w - pp * (PL::NSAB * 4);
+        const int m = rest >> 2, row = rest & 3;
+        const int ma = m / PL::NSB, mb = m - ma * PL::NSB;
+        const int pp0 = s_src[pp];
         const int i = pp0 / B.nprim, j = pp0 % B.nprim;
         const double a = exps[A.prim + i], b = exps[B.prim + j];
         const double p = a + b;
         const double mu = a * b / p;
         const double px = (a * A.x + b * B.x) / p, py = (a * A.y + b * B.y) / p, pz = (a * A.z + b * B.z) / p;
         double* s = smem + pp * PL::STRIDE;
-        s[0] = p;
-        s[1] = px;
-        s[2] = py;
-        s[3] = pz;
+        if (rest == 0) {
+            s[0] = p;
+            s[1] = px;
+            s[2] = py;
+            s[3] = pz;
+            s[PL::INV] = 1.0 / p;
 #pragma unroll
-        for (int ka = 0; ka < PL::KA; ++ka)
+            for (int ka = 0; ka < PL::KA; ++ka)
 #pragma unroll
-            for (int kb = 0; kb < PL::KB; ++kb)
-                s[4 + ka * PL::KB + kb] = (ka < A.ncontr && kb < B.ncontr)
-                                              ? coefs[A.coef + ka * A.nprim + i] * coefs[B.coef + kb * B.nprim + j]
-                                              : 0.0;
+                for (int kb = 0; kb < PL::KB; ++kb)
+                    s[PL::CC + ka * PL::KB + kb] =
+                        (ka < A.ncontr && kb < B.ncontr)
+                            ? coefs[A.coef + ka * A.nprim + i] * coefs[B.coef + kb * B.nprim + j]
+                            : 0.0;
+        }
         Hermite1D<LA + 1, LB> ex, ey, ez;
         ex.build(p, exp(-mu * rab2), px - A.x, px - B.x);
         ey.build(p, 1.0, py - A.y, py - B.y);
         ez.build(p, 1.0, pz - A.z, pz - B.z);
-        double* et = s + PL::OFF_E;
-        double* ea = s + PL::OFF_EA;
-        for (int k = 0; k < PL::NSAB * PL::NH; ++k) et[k] = 0.0;
-        for (int k = 0; k < 3 * PL::NSAB * PL::NH1; ++k) ea[k] = 0.0;
+        const int d = row - 1;  // -1: values
+        const int nh = row == 0 ? PL::NH : PL::NH1;
+        double* et = row == 0 ? s + PL::OFF_E + m * PL::NH : s + PL::OFF_EA + (d * PL::NSAB + m) * PL::NH1;
+        for (int h = 0; h < nh; ++h) et[h] = 0.0;
+        // one axis: E^{ij}_t, or along d its derivative by the first centre, 2a E^{i+1,j}_t - i E^{i-1,j}_t
+        auto axis = [&](const Hermite1D<LA + 1, LB>& e, bool raised, int ii, int jj, int t) {
+            if (!raised) return e.e[ii][jj][t];
+            return 2.0 * a * e.e[ii + 1][jj][t] - (ii > 0 ? ii * e.e[ii - 1][jj][t] : 0.0);
+        };
 #pragma unroll 1
-        for (int ca = 0; ca < NCA; ++ca)
+        for (int ca = 0; ca < NCA; ++ca) {
+            const double ra = c_c2s[c2s_offset(LA) + ma * NCA + ca];
+            if (ra == 0.0) continue;
 #pragma unroll 1
             for (int cb = 0; cb < NCB; ++cb) {
+                const double w2 = ra * c_c2s[c2s_offset(LB) + mb * NCB + cb];
+                if (w2 == 0.0) continue;
                 const int ix = c_cart[LA][ca][0], iy = c_cart[LA][ca][1], iz = c_cart[LA][ca][2];
                 const int jx = c_cart[LB][cb][0], jy = c_cart[LB][cb][1], jz = c_cart[LB][cb][2];
-                // value: E^{ij}_t per axis
 #pragma unroll 1
-                for (int t = 0; t <= ix + jx; ++t)
+                for (int t = 0; t <= ix + jx + (d == 0); ++t) {
+                    const double fx = axis(ex, d == 0, ix, jx, t);
 #pragma unroll 1
-                    for (int u = 0; u <= iy + jy; ++u)
+                    for (int u = 0; u <= iy + jy + (d == 1); ++u) {
+                        const double fy = axis(ey, d == 1, iy, jy, u);
 #pragma unroll 1
-                        for (int v = 0; v <= iz + jz; ++v) {
-                            const double w = ex.e[ix][jx][t] * ey.e[iy][jy][u] * ez.e[iz][jz][v];
-#pragma unroll 1
-                            for (int ma = 0; ma < PL::NSA; ++ma) {
-                                const double wa = c_c2s[c2s_offset(LA) + ma * NCA + ca] * w;
-                                if (wa == 0.0) continue;
-#pragma unroll 1
-                                for (int mb = 0; mb < PL::NSB; ++mb)
-                                    et[(ma * PL::NSB + mb) * PL::NH + tet(t, u, v)] +=
-                                        c_c2s[c2s_offset(LB) + mb * NCB + cb] * wa;
-                            }
-                        }
-                // derivative by the first centre along each axis: 2a E^{i+1,j} - i E^{i-1,j}
-#pragma unroll 1
-                for (int d = 0; d < 3; ++d) {
-                    const int ext = 1;
-#pragma unroll 1
-                    for (int t = 0; t <= ix + jx + (d == 0 ? ext : 0); ++t) {
-                        const double fx = d == 0 ? 2.0 * a * ex.e[ix + 1][jx][t] - (ix > 0 ? ix * ex.e[ix - 1][jx][t] : 0.0)
-                                                 : (t <= ix + jx ? ex.e[ix][jx][t] : 0.0);
-                        if (fx == 0.0) continue;
-#pragma unroll 1
-                        for (int u = 0; u <= iy + jy + (d == 1 ? ext : 0); ++u) {
-                            const double fy = d == 1 ? 2.0 * a * ey.e[iy + 1][jy][u] - (iy > 0 ? iy * ey.e[iy - 1][jy][u] : 0.0)
-                                                     : (u <= iy + jy ? ey.e[iy][jy][u] : 0.0);
-                            if (fy == 0.0) continue;
-#pragma unroll 1
-                            for (int v = 0; v <= iz + jz + (d == 2 ? ext : 0); ++v) {
-                                const double fz = d == 2 ? 2.0 * a * ez.e[iz + 1][jz][v] - (iz > 0 ? iz * ez.e[iz - 1][jz][v] : 0.0)
-                                                         : (v <= iz + jz ? ez.e[iz][jz][v] : 0.0);
-                                const double w = fx * fy * fz;
-                                if (w == 0.0) continue;
-#pragma unroll 1
-                                for (int ma = 0; ma < PL::NSA; ++ma) {
-                                    const double wa = c_c2s[c2s_offset(LA) + ma * NCA + ca] * w;
-                                    if (wa == 0.0) continue;
-#pragma unroll 1
-                                    for (int mb = 0; mb < PL::NSB; ++mb)
-                                        ea[(d * PL::NSAB + ma * PL::NSB + mb) * PL::NH1 + tet(t, u, v)] +=
-                                            c_c2s[c2s_offset(LB) + mb * NCB + cb] * wa;
-                                }
-                            }
-                        }
+                        for (int v = 0; v <= iz + jz + (d == 2); ++v)
+                            et[tet(t, u, v)] += w2 * fx * fy * axis(ez, d == 2, iz, jz, v);
                     }
                 }
             }
-        // the Coulomb weight's orbital part: DJ[m] = sum_k cc[k] D[mu_k,m][nu_k,m]
-        double dj[PL::NSAB];
-#pragma unroll
-        for (int m = 0; m < PL::NSAB; ++m) dj[m] = 0.0;
-        for (int ka = 0; ka < A.ncontr; ++ka)
-            for (int kb = 0; kb < B.ncontr; ++kb) {
-                const double c = s[4 + ka * PL::KB + kb];
-#pragma unroll
-                for (int ma = 0; ma < PL::NSA; ++ma)
-#pragma unroll
-                    for (int mb = 0; mb < PL::NSB; ++mb)
-                        dj[ma * PL::NSB + mb] +=
-                            c * D[(int64_t)(A.fn + ka * PL::NSA + ma) * n + B.fn + kb * PL::NSB + mb];
-            }
-        double* ej = s + PL::OFF_EJ;
-        double* eja = s + PL::OFF_EJA;
-        for (int h = 0; h < PL::NH; ++h) {
-            double acc = 0.0;
-#pragma unroll
-            for (int m = 0; m < PL::NSAB; ++m) acc += dj[m] * et[m * PL::NH + h];
-            ej[h] = acc;
         }
-        for (int k = 0; k < 3 * PL::NH1; ++k) {
-            const int d = k / PL::NH1, h = k % PL::NH1;
-            double acc = 0.0;
-#pragma unroll
-            for (int m = 0; m < PL::NSAB; ++m) acc += dj[m] * ea[(d * PL::NSAB + m) * PL::NH1 + h];
-            eja[k] = acc;
+    }
+    __syncthreads();
+    // the Coulomb weight's orbital part: DJ[m] = sum_k cc[k] D[mu_k,m][nu_k,m], then EJ = DJ . E and
+    // EJA = DJ . EA, one task per entry
+    constexpr int NJ = PL::NH + 3 * PL::NH1;
+    for (int w = threadIdx.x; w < nk * NJ; w += blockDim.x) {
+        const int pp = w / NJ, h = w - pp * NJ;
+        double* s = smem + pp * PL::STRIDE;
+        const int k = h - PL::NH, d = k < 0 ? 0 : k / PL::NH1;
+        const double* e = k < 0 ? s + PL::OFF_E + h : s + PL::OFF_EA + d * PL::NSAB * PL::NH1 + (k - d * PL::NH1);
+        const int stride = k < 0 ? PL::NH : PL::NH1;
+        double acc = 0.0;
+#pragma unroll 1
+        for (int m = 0; m < PL::NSAB; ++m) {
+            const int ma = m / PL::NSB, mb = m - ma * PL::NSB;
+            double dj = 0.0;
+            for (int ka = 0; ka < A.ncontr; ++ka)
+                for (int kb = 0; kb < B.ncontr; ++kb)
+                    dj += s[PL::CC + ka * PL::KB + kb] *
+                          D[(int64_t)(A.fn + ka * PL::NSA + ma) * n + B.fn + kb * PL::NSB + mb];
+            acc += dj * e[m * stride];
         }
+        (k < 0 ? s + PL::OFF_EJ : s + PL::OFF_EJA - PL::NH)[h] = acc;
     }
     __syncthreads();
     return s_pos[kMaxPrimPairs];
@@ -227,7 +203,7 @@ __global__ void __launch_bounds__(kGradThreads) k_grad_pair_data(const PairTask*
                                                                  double* __restrict__ data, int* __restrict__ npps) {
     using PL = GradPairLayout<LA, LB>;
     extern __shared__ double smem[];
-    __shared__ int s_pos[kMaxPrimPairs + 1];
+    __shared__ int s_pos[2 * kMaxPrimPairs + 1];
     const PairTask task = tasks[blockIdx.x];
     const DevShell A = orb[task.swap ? task.second : task.first];
     const DevShell B = orb[task.swap ? task.first : task.second];
@@ -388,16 +364,15 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
                 if (ti != ci) {
                     ci = ti;
                     q = exps[P.prim + ti];
-                    // c_P (2q)^-l_P (-1)^l_P
-                    const double h2q = 0.5 / q;
-                    cq = coefs[P.coef + ti];
-#pragma unroll
-                    for (int k = 0; k < LP; ++k) cq *= h2q;
+                    // c_P (2q)^-l_P (-1)^l_P 2 pi^(5/2) / q
+                    const double inv_q = 1.0 / q;
+                    cq = coefs[P.coef + ti] * half_power<LP>(inv_q) * kTwoPi52 * inv_q;
                     if (LP & 1) cq = -cq;
                 }
                 const double* s = pd + (int64_t)pp * PL::STRIDE;
                 const double p = s[0];
-                const double inv_pq = 1.0 / (p + q);
+                double inv_pq, inv_root;
+                inverse_sum(p, q, inv_pq, inv_root);
                 const double alpha = p * q * inv_pq;
                 double* row = sR + (slot * TPR + mp) * RS;
                 if constexpr (L <= 4) {
@@ -409,7 +384,7 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
                     hermite_r<L>(alpha, s[1] - P.x, s[2] - P.y, s[3] - P.z, btable, row);
                 }
                 // 2 pi^(5/2) / (p q sqrt(p + q)) c_P (2q)^-l_P (-1)^l_P
-                row[NR] = kTwoPi52 * sqrt(inv_pq) / (p * q) * cq;
+                row[NR] = inv_root * s[PL::INV] * cq;
                 tpp += TPR;
                 while (tpp >= npp) {
                     tpp -= npp;
@@ -433,7 +408,7 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
                 for (int m = 0; m < PL::NSAB; ++m) {
                     double x = 0.0;
 #pragma unroll
-                    for (int k = 0; k < PL::KK; ++k) x += s[4 + k] * gk[k][m];
+                    for (int k = 0; k < PL::KK; ++k) x += s[PL::CC + k] * gk[k][m];
                     w[m] = x;
                 }
                 const double* et = s + PL::OFF_E;
@@ -531,12 +506,12 @@ cudaError_t launch_three_center_grad(int la, int lb, const PairTask* tasks, int 
                                      const DevShell* orb, const DevShell* aux, const double* exps,
                                      const double* coefs, const int* const* alist_by_l, const int* count_by_l,
                                      const double* btable, GradWeights g, GradPairData pd, double* gorb,
-                                     double* gaux, cudaStream_t stream) {
+                                     double* gaux, Branches& br) {
     cudaError_t e = cudaSuccess;
 #define HF_3CG(LA, LB, LP)                                                                                        \
     if (e == cudaSuccess && la == LA && lb == LB)                                                                 \
         e = three_center_grad_one<LA, LB, LP>(tasks, ntasks, max_npp, orb, aux, exps, coefs, alist_by_l[LP],       \
-                                              count_by_l[LP], btable, g, pd, gorb, gaux, stream);
+                                              count_by_l[LP], btable, g, pd, gorb, gaux, br.next());
 #define HF_3CG_P(LA, LB) HF_3CG(LA, LB, 0) HF_3CG(LA, LB, 1) HF_3CG(LA, LB, 2) HF_3CG(LA, LB, 3) HF_3CG(LA, LB, 4)
     HF_3CG_P(0, 0)
     HF_3CG_P(0, 1)
@@ -620,15 +595,18 @@ __global__ void __launch_bounds__(128) k_metric_grad(const DevShell* __restrict_
             for (int m = 0; m < NSQ; ++m) val[d][m] = 0.0;
         for (int i = 0; i < P.nprim; ++i) {
             const double p = exps[P.prim + i];
-            const double cp = coefs[P.coef + i] * pow(2.0 * p, -(double)LP);
+            const double inv_p = 1.0 / p;
+            const double cp = coefs[P.coef + i] * half_power<LP>(inv_p) * kTwoPi52 * inv_p;
             for (int j = 0; j < Q.nprim; ++j) {
                 const double q = exps[Q.prim + j];
-                double cq = coefs[Q.coef + j] * pow(2.0 * q, -(double)LQ);
+                const double inv_q = 1.0 / q;
+                double cq = coefs[Q.coef + j] * half_power<LQ>(inv_q) * inv_q;
                 if (LQ & 1) cq = -cq;
-                const double alpha = p * q / (p + q);
+                double inv_pq, inv_root;
+                inverse_sum(p, q, inv_pq, inv_root);
                 double R[ntet(L)];
-                hermite_r<L>(alpha, X, Y, Z, btable, R);
-                const double pref = kTwoPi52 / (p * q * sqrt(p + q)) * cp * cq;
+                hermite_r<L>(p * q * inv_pq, X, Y, Z, btable, R);
+                const double pref = inv_root * cp * cq;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     double h[NCQ];
@@ -688,12 +666,12 @@ static cudaError_t metric_grad_one(const DevShell* aux, const double* exps, cons
 
 cudaError_t launch_metric_grad(const DevShell* aux, const double* exps, const double* coefs,
                                const int* const* aux_by_l, const int* count, const double* btable, const double* WJ,
-                               const double* WK, int64_t ldw, double* gaux, cudaStream_t stream) {
+                               const double* WK, int64_t ldw, double* gaux, Branches& br) {
     cudaError_t e = cudaSuccess;
 #define HF_MG(LP, LQ)                                                                                            \
     if (e == cudaSuccess)                                                                                        \
         e = metric_grad_one<LP, LQ>(aux, exps, coefs, aux_by_l[LP], count[LP], aux_by_l[LQ], count[LQ], btable, WJ, \
-                                    WK, ldw, gaux, stream);
+                                    WK, ldw, gaux, br.next());
 #define HF_MG_ROW(LP) HF_MG(LP, 0) HF_MG(LP, 1) HF_MG(LP, 2) HF_MG(LP, 3) HF_MG(LP, 4)
     HF_MG_ROW(0)
     HF_MG_ROW(1)
@@ -743,8 +721,9 @@ __device__ __forceinline__ void cartesian_weights(const DevShell& A, const DevSh
         }
 }
 
-// One thread per ordered shell pair (A, B) of class (LA, LB): <d_A u|T + V|v>
-// against D (slots 0..2, times 2 for the ket by symmetry) and -<d_A u|v> against
+// One warp per ordered shell pair (A, B) of class (LA, LB): groups of lanes take
+// the primitive pairs in turn, the lanes of a group share the sum over the nuclei
+// (a thread per pair ran all of both sums in one chain). <d_A u|T + V|v> against D (slots 0..2, times 2 for the ket by symmetry) and -<d_A u|v> against
 // W (slots 3..5, times -2) into gorb[A] (gradient.py:171-178, 119-124).
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) k_one_electron_grad(const int2* __restrict__ tasks, int ntasks,
@@ -759,19 +738,26 @@ __global__ void __launch_bounds__(128) k_one_electron_grad(const int2* __restric
     constexpr int NCA = ncart(LA), NCB = ncart(LB);
     constexpr int KA = kMaxOrbContr[LA], KB = kMaxOrbContr[LB];
     constexpr int LAB = LA + LB;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntasks) return;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (t >= ntasks) return;  // whole warps
     const int2 task = tasks[t];
     const DevShell A = orb[task.x];
     const DevShell B = orb[task.y];
+    const int npp = A.nprim * B.nprim;
+    int share = 1;  // lanes per primitive pair
+    while (share < 32 && share * npp * 2 <= 32) share *= 2;
+    const int sub = lane & (share - 1);
     double dc[KA * KB][NCA][NCB], wc[KA * KB][NCA][NCB];
     cartesian_weights<LA, LB>(A, B, D, n, dc);
     cartesian_weights<LA, LB>(A, B, W, n, wc);
     double g1[3] = {0.0, 0.0, 0.0}, gs[3] = {0.0, 0.0, 0.0};
     const double abx = A.x - B.x, aby = A.y - B.y, abz = A.z - B.z;
     const double rab2 = abx * abx + aby * aby + abz * abz;
-    for (int i = 0; i < A.nprim; ++i)
-        for (int j = 0; j < B.nprim; ++j) {
+    const int rounds = (npp * share + 31) / 32;
+    for (int r = 0; r < rounds; ++r) {
+            const int pp = (r * 32 + lane) / share;
+            const bool on = pp < npp;
+            const int i = on ? pp / B.nprim : 0, j = on ? pp - i * B.nprim : 0;
             const double a = exps[A.prim + i], b = exps[B.prim + j];
             const double p = a + b, mu = a * b / p;
             const double px = (a * A.x + b * B.x) / p, py = (a * A.y + b * B.y) / p, pz = (a * A.z + b * B.z) / p;
@@ -782,7 +768,7 @@ __global__ void __launch_bounds__(128) k_one_electron_grad(const int2* __restric
             double Rs[ntet(LAB + 1)];
 #pragma unroll
             for (int h = 0; h < ntet(LAB + 1); ++h) Rs[h] = 0.0;
-            for (int c = 0; c < natoms; ++c) {
+            for (int c = on ? sub : natoms; c < natoms; c += share) {
                 double R[ntet(LAB + 1)];
                 hermite_r<LAB + 1>(p, px - positions[3 * c], py - positions[3 * c + 1], pz - positions[3 * c + 2],
                                    btable, R);
@@ -790,7 +776,12 @@ __global__ void __launch_bounds__(128) k_one_electron_grad(const int2* __restric
 #pragma unroll
                 for (int h = 0; h < ntet(LAB + 1); ++h) Rs[h] -= z * R[h];
             }
-            const double ov = pow(kPi / p, 1.5);
+            __syncwarp();
+            for (int o = share >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int h = 0; h < ntet(LAB + 1); ++h) Rs[h] += __shfl_xor_sync(0xffffffffu, Rs[h], o);
+            if (!on || sub != 0) continue;
+            const double ov = kPi / p * sqrt(kPi / p);
             const double vpref = 2.0 * kPi / p;
             // per-primitive density weights
             double cf[KA * KB];
@@ -864,6 +855,15 @@ __global__ void __launch_bounds__(128) k_one_electron_grad(const int2* __restric
                     }
                 }
         }
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            g1[d] += __shfl_xor_sync(0xffffffffu, g1[d], o);
+            gs[d] += __shfl_xor_sync(0xffffffffu, gs[d], o);
+        }
+    if (lane != 0) return;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         atomicAdd(gorb + (int64_t)task.x * 6 + d, 2.0 * g1[d]);
@@ -957,14 +957,14 @@ template <int LA, int LB>
 static cudaError_t one_electron_grad_one(const int2* tasks, int ntasks, const DevShell* orb, const double* exps,
                                          const double* coefs, const double* charges, const double* positions,
                                          int natoms, const double* btable, const double* D, const double* W, int64_t n,
-                                         double* gorb, double* gatom, cudaStream_t stream) {
+                                         double* gorb, double* gatom, Branches& br) {
     if (ntasks == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((ntasks + 127) / 128);
-    k_one_electron_grad<LA, LB><<<blocks, 128, 0, stream>>>(tasks, ntasks, orb, exps, coefs, charges, positions, natoms,
+    k_one_electron_grad<LA, LB><<<(unsigned)((ntasks + 3) / 4), 128, 0, br.next()>>>(tasks, ntasks, orb, exps, coefs, charges, positions, natoms,
                                                             btable, D, W, n, gorb);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || natoms == 0) return e;
-    k_attraction_nucleus_grad<LA, LB><<<dim3(blocks, natoms), 128, 0, stream>>>(tasks, ntasks, orb, exps, coefs, charges,
+    k_attraction_nucleus_grad<LA, LB><<<dim3(blocks, natoms), 128, 0, br.next()>>>(tasks, ntasks, orb, exps, coefs, charges,
                                                                                positions, btable, D, n, gatom);
     return cudaGetLastError();
 }
@@ -972,12 +972,12 @@ static cudaError_t one_electron_grad_one(const int2* tasks, int ntasks, const De
 cudaError_t launch_one_electron_grad(int la, int lb, const int2* tasks, int ntasks, const DevShell* orb,
                                      const double* exps, const double* coefs, const double* charges,
                                      const double* positions, int natoms, const double* btable, const double* D,
-                                     const double* W, int64_t n, double* gorb, double* gatom, cudaStream_t stream) {
+                                     const double* W, int64_t n, double* gorb, double* gatom, Branches& br) {
     cudaError_t e = cudaSuccess;
 #define HF_1EG(LA, LB)                                                                                        \
     if (la == LA && lb == LB)                                                                                 \
         e = one_electron_grad_one<LA, LB>(tasks, ntasks, orb, exps, coefs, charges, positions, natoms, btable, D, W, \
-                                          n, gorb, gatom, stream);
+                                          n, gorb, gatom, br);
     HF_1EG(0, 0) HF_1EG(0, 1) HF_1EG(0, 2) HF_1EG(1, 0) HF_1EG(1, 1) HF_1EG(1, 2) HF_1EG(2, 0) HF_1EG(2, 1)
     HF_1EG(2, 2)
 #undef HF_1EG

@@ -120,7 +120,7 @@ std::vector<double> boys_grid_host() {
     static std::vector<double> cached;
     std::lock_guard<std::mutex> lock(mutex);
     if (!cached.empty()) return cached;
-    std::vector<double> g(kBoysGrid * kBoysOrders);
+    std::vector<double> g(kBoysGrid * kBoysStride);
     const int nmax = kBoysOrders - 1;
     for (int j = 0; j < kBoysGrid; ++j) {
         const double t = j * kBoysStep;
@@ -131,8 +131,9 @@ std::vector<double> boys_grid_host() {
             sum += term;
             if (term < sum * 1e-17) break;
         }
-        double* row = &g[j * kBoysOrders];
+        double* row = &g[j * kBoysStride];
         row[nmax] = et * sum;
+        row[kBoysOrders] = et;
         for (int n = nmax; n >= 1; --n) row[n - 1] = (2.0 * t * row[n] + et) / (2 * n - 1);
     }
     cached = g;
@@ -203,15 +204,18 @@ __global__ void __launch_bounds__(128) k_metric(const DevShell* __restrict__ aux
     const double X = P.x - Q.x, Y = P.y - Q.y, Z = P.z - Q.z;
     for (int i = 0; i < P.nprim; ++i) {
         const double p = exps[P.prim + i];
-        const double cp = coefs[P.coef + i] * pow(2.0 * p, -(double)LP);
+        const double inv_p = 1.0 / p;
+        const double cp = coefs[P.coef + i] * half_power<LP>(inv_p) * kTwoPi52 * inv_p;
         for (int j = 0; j < Q.nprim; ++j) {
             const double q = exps[Q.prim + j];
-            double cq = coefs[Q.coef + j] * pow(2.0 * q, -(double)LQ);
+            const double inv_q = 1.0 / q;
+            double cq = coefs[Q.coef + j] * half_power<LQ>(inv_q) * inv_q;
             if (LQ & 1) cq = -cq;
-            const double alpha = p * q / (p + q);
+            double inv_pq, inv_root;
+            inverse_sum(p, q, inv_pq, inv_root);
             double R[ntet(L)];
-            hermite_r<L>(alpha, X, Y, Z, btable, R);
-            const double pref = kTwoPi52 / (p * q * sqrt(p + q)) * cp * cq;
+            hermite_r<L>(p * q * inv_pq, X, Y, Z, btable, R);
+            const double pref = inv_root * cp * cq;  // 2 pi^(5/2) / (p q sqrt(p + q)) and the coefficients
             double h[NCQ];
 #pragma unroll
             for (int b = 0; b < NCQ; ++b) {
@@ -249,12 +253,12 @@ static cudaError_t metric_one(const DevShell* aux, const double* exps, const dou
 
 cudaError_t launch_metric(const DevShell* aux, const double* exps, const double* coefs,
                           const int* const* aux_by_l, const int* count, const double* btable, double* M,
-                          int64_t ldm, cudaStream_t stream) {
+                          int64_t ldm, Branches& br) {
     cudaError_t e = cudaSuccess;
 #define HF_METRIC(LP, LQ)                                                                                    \
     if (e == cudaSuccess)                                                                                    \
         e = metric_one<LP, LQ>(aux, exps, coefs, aux_by_l[LP], count[LP], aux_by_l[LQ], count[LQ], btable, M, \
-                               ldm, stream);
+                               ldm, br.next());
 #define HF_METRIC_ROW(LP) HF_METRIC(LP, 0) HF_METRIC(LP, 1) HF_METRIC(LP, 2) HF_METRIC(LP, 3) HF_METRIC(LP, 4)
     HF_METRIC_ROW(0)
     HF_METRIC_ROW(1)
@@ -376,6 +380,56 @@ __device__ int pair_prologue(const DevShell& A, const DevShell& B, const double*
     return nk;
 }
 
+// The pair data of pair_prologue, built once per shell pair into global memory (stride doubles per
+// task) for every auxiliary class and slab: a CTA per (pair, slab) that builds it itself spends most
+// of its time on it for the high classes, whose pairs have few primitives and whose slabs are many.
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) k_pair_data(const PairTask* __restrict__ tasks, const DevShell* __restrict__ orb,
+                                                   const double* __restrict__ exps, const double* __restrict__ coefs,
+                                                   double* __restrict__ data, int64_t stride, int* __restrict__ npps) {
+    extern __shared__ double smem[];
+    __shared__ int s_pos[2 * kMaxPrimPairs + 1];
+    const PairTask task = tasks[blockIdx.x];
+    const DevShell A = orb[task.swap ? task.second : task.first];
+    const DevShell B = orb[task.swap ? task.first : task.second];
+    const int npp = pair_prologue<LA, LB>(A, B, exps, coefs, smem, s_pos);  // ends with a barrier
+    double* dst = data + (int64_t)blockIdx.x * stride;
+    for (int k = threadIdx.x; k < npp * PairLayout<LA, LB>::STRIDE; k += blockDim.x) dst[k] = smem[k];
+    if (threadIdx.x == 0) npps[blockIdx.x] = npp;
+}
+
+template <int LA, int LB>
+static cudaError_t pair_data_one(const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
+                                 const double* exps, const double* coefs, PairData pd, cudaStream_t stream) {
+    const size_t smem = sizeof(double) * (size_t)max_npp * PairLayout<LA, LB>::STRIDE;
+    if (smem > 40 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k_pair_data<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    k_pair_data<LA, LB><<<ntasks, 128, smem, stream>>>(tasks, orb, exps, coefs, pd.data, pd.stride, pd.npps);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pair_data(int la, int lb, const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
+                             const double* exps, const double* coefs, PairData pd, cudaStream_t stream) {
+    cudaError_t e = cudaSuccess;
+    if (ntasks == 0) return e;
+#define HF_PD(LA, LB) \
+    if (la == LA && lb == LB) e = pair_data_one<LA, LB>(tasks, ntasks, max_npp, orb, exps, coefs, pd, stream);
+    HF_PD(0, 0) HF_PD(0, 1) HF_PD(0, 2) HF_PD(1, 1) HF_PD(1, 2) HF_PD(2, 2)
+#undef HF_PD
+    return e;
+}
+
+int64_t pair_data_stride(int la, int lb, int max_npp) {
+    int64_t stride = 0;
+#define HF_STRIDE(LA, LB) \
+    if (la == LA && lb == LB) stride = PairLayout<LA, LB>::STRIDE;
+    HF_STRIDE(0, 0) HF_STRIDE(0, 1) HF_STRIDE(0, 2) HF_STRIDE(1, 1) HF_STRIDE(1, 2) HF_STRIDE(2, 2)
+#undef HF_STRIDE
+    return stride * max_npp;
+}
+
 // Shapes of one (P|mu nu) class. The threads of an auxiliary shell (one per
 // m_P, all in one warp) share each primitive triple's R table: per round, TPR
 // of them each evaluate the Boys function and R table of one triple into
@@ -414,19 +468,25 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
                                                       const double* __restrict__ coefs,
                                                       const int* __restrict__ alist, int nalist,
                                                       const double* __restrict__ btable, ChunkDesc chunk,
-                                                      int r_offset, double* __restrict__ T) {
+                                                      const double* __restrict__ pdata, int64_t pstride,
+                                                      const int* __restrict__ npps, int r_offset,
+                                                      double* __restrict__ T) {
     using PL = PairLayout<LA, LB>;
     using SH = ThreeCenterShape<LA, LB, LP>;
     constexpr int L = SH::L, NCP = SH::NCP, NSP = SH::NSP, SPW = SH::SPW, NH = SH::NH, TPR = SH::TPR;
     constexpr int RS = SH::RS, NR = SH::NR;
     extern __shared__ double smem[];
-    __shared__ int s_pos[2 * kMaxPrimPairs + 1];
     __shared__ int s_idx[NCP * NH];      // tet(h + c) for Cartesian c of l_P, Hermite h of the pair
     __shared__ int s_nzc[NSP * NCP];     // per m_P: the Cartesian components with a nonzero weight
     __shared__ double s_nzw[NSP * NCP];  // ... and the weights
     __shared__ int s_nnz[NSP];
     __shared__ int s_tp[SH::SPB * TPR];  // primitive pair of each table of the round, -1 past the end
     double* sR = smem + r_offset;
+    const PairTask task = tasks[blockIdx.x];
+    const int npp = npps[blockIdx.x];
+    if (npp == 0) return;  // the same for the whole CTA; the chunk was zeroed
+    const double* __restrict__ pd = pdata + (int64_t)blockIdx.x * pstride;
+    for (int e = threadIdx.x; e < npp * PL::STRIDE; e += blockDim.x) smem[e] = pd[e];
 
     for (int e = threadIdx.x; e < NCP * NH; e += blockDim.x) {
         const int c = e / NH, h = e - c * NH;
@@ -445,11 +505,9 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
         s_nnz[threadIdx.x] = k;
     }
 
-    const PairTask task = tasks[blockIdx.x];
+    __syncthreads();
     const DevShell A = orb[task.swap ? task.second : task.first];
     const DevShell B = orb[task.swap ? task.first : task.second];
-    const int npp = pair_prologue<LA, LB>(A, B, exps, coefs, smem, s_pos);  // ends with a barrier
-    if (npp == 0) return;  // the same for the whole CTA; the chunk was zeroed
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wslot = lane / NSP, mp = lane - wslot * NSP;
@@ -495,11 +553,11 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
             }
             const double* s = smem + pp * PL::STRIDE;
             const double p = s[0];
-            // one division per primitive triple: 1/(p+q) gives both the reduced
-            // exponent and the prefactor 2 pi^(5/2) / (p q sqrt(p+q))
-            const double inv_pq = 1.0 / (p + q);
+            // the reduced exponent and the prefactor 2 pi^(5/2) / (p q sqrt(p+q))
+            double inv_pq, inv_root;
+            inverse_sum(p, q, inv_pq, inv_root);
             const double alpha = p * q * inv_pq;
-            const double pref = s[4] * sqrt(inv_pq) * cq;
+            const double pref = s[4] * inv_root * cq;
             if constexpr (NSP == 1) {
                 hermite_r<L>(alpha, s[1] - P.x, s[2] - P.y, s[3] - P.z, btable, R);
                 const double scale = pref * c_c2s[c2s_offset(LP)];  // the single weight of l_P = 0
@@ -616,7 +674,7 @@ template <int LA, int LB, int LP>
 static cudaError_t three_center_one(const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
                                     const DevShell* aux, const double* exps, const double* coefs,
                                     const int* alist, int nalist, const double* btable, ChunkDesc chunk,
-                                    double* T, cudaStream_t stream) {
+                                    PairData pd, double* T, cudaStream_t stream) {
     if (ntasks == 0 || nalist == 0) return cudaSuccess;
     using SH = ThreeCenterShape<LA, LB, LP>;
     const int r_offset = max_npp * PairLayout<LA, LB>::STRIDE;
@@ -630,19 +688,19 @@ static cudaError_t three_center_one(const PairTask* tasks, int ntasks, int max_n
     }
     dim3 grid(ntasks, (nalist + SH::SPB - 1) / SH::SPB);  // 4 warps of SPW shells
     k_three_center<LA, LB, LP><<<grid, 128, smem, stream>>>(tasks, orb, aux, exps, coefs, alist, nalist, btable,
-                                                            chunk, r_offset, T);
+                                                            chunk, pd.data, pd.stride, pd.npps, r_offset, T);
     return cudaGetLastError();
 }
 
 cudaError_t launch_three_center(int la, int lb, const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
                                 const DevShell* aux, const double* exps, const double* coefs,
                                 const int* const* aux_by_l, const int* count, const double* btable,
-                                ChunkDesc chunk, double* T, cudaStream_t stream) {
+                                ChunkDesc chunk, PairData pd, double* T, Branches& br) {
     cudaError_t e = cudaSuccess;
 #define HF_3C(LA, LB, LP)                                                                                     \
     if (e == cudaSuccess && la == LA && lb == LB)                                                             \
         e = three_center_one<LA, LB, LP>(tasks, ntasks, max_npp, orb, aux, exps, coefs, aux_by_l[LP], count[LP], \
-                                         btable, chunk, T, stream);
+                                         btable, chunk, pd, T, br.next());
 #define HF_3C_P(LA, LB) HF_3C(LA, LB, 0) HF_3C(LA, LB, 1) HF_3C(LA, LB, 2) HF_3C(LA, LB, 3) HF_3C(LA, LB, 4)
     HF_3C_P(0, 0)
     HF_3C_P(0, 1)
@@ -731,7 +789,7 @@ __global__ void __launch_bounds__(128) k_one_electron(const int2* __restrict__ t
                         cart[ca][cb] = pref * s;
                     }
             } else {
-                const double ov = pow(kPi / p, 1.5);
+                const double ov = kPi / p * sqrt(kPi / p);
 #pragma unroll
                 for (int ca = 0; ca < NCA; ++ca)
 #pragma unroll

@@ -35,10 +35,39 @@ struct PairTask {
     int first, second, swap, pad;
 };
 
-struct ShellClassLists {
-    // orbital pairs bucketed by (la, lb) with la <= lb: 3x3 buckets (only la<=lb used)
-    std::vector<PairTask> pairs[3][3];
-    int max_npp[3][3] = {};
+// Hermite data of one class's pair tasks (launch_pair_data).
+struct PairData {
+    double* data;
+    int64_t stride;  // doubles per task
+    int* npps;
+};
+
+// The launches of independent classes, spread over side streams so that classes
+// too small to fill the chip run beside one another: fork() orders the side
+// streams after the work of `main`, next() names the stream of the next launch,
+// join() orders `main` after all of them.
+struct Branches {
+    static constexpr int kCount = 6;
+    cudaStream_t main = nullptr;
+    cudaStream_t side[kCount] = {};
+    cudaEvent_t event[kCount + 1] = {};
+    bool have = false;
+    int at = 0;
+    cudaStream_t next() { return have ? side[at++ % kCount] : main; }
+    cudaError_t fork() {
+        if (!have) return cudaSuccess;
+        cudaError_t e = cudaEventRecord(event[kCount], main);
+        for (int i = 0; i < kCount && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(side[i], event[kCount], 0);
+        return e;
+    }
+    cudaError_t join() {
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; have && i < kCount && e == cudaSuccess; ++i) {
+            e = cudaEventRecord(event[i], side[i]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(main, event[i], 0);
+        }
+        return e;
+    }
 };
 
 // The constant tables every integral kernel reads (each translation unit with
@@ -64,13 +93,19 @@ cudaError_t launch_boys_values(const double* t, int64_t count, int n_max, const 
 // (P|Q) for all aux shells into M[N][N] (internal order, row-major, ld = ldm).
 cudaError_t launch_metric(const DevShell* aux, const double* exps, const double* coefs,
                           const int* const* aux_by_l_dev, const int* aux_count, const double* btable,
-                          double* M, int64_t ldm, cudaStream_t stream);
+                          double* M, int64_t ldm, Branches& br);
 
 // (P|ab) for the given pair tasks of class (la, lb) and all aux shells, into a chunk.
 cudaError_t launch_three_center(int la, int lb, const PairTask* tasks, int ntasks, int max_npp,
                                 const DevShell* orb, const DevShell* aux, const double* exps,
                                 const double* coefs, const int* const* aux_by_l_dev, const int* aux_count,
-                                const double* btable, ChunkDesc chunk, double* T, cudaStream_t stream);
+                                const double* btable, ChunkDesc chunk, PairData pd, double* T, Branches& br);
+
+// The pair tasks' Hermite data for launch_three_center: stride =
+// pair_data_stride(la, lb, max_npp) doubles per task, npps[task] primitive pairs kept.
+cudaError_t launch_pair_data(int la, int lb, const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
+                             const double* exps, const double* coefs, PairData pd, cudaStream_t stream);
+int64_t pair_data_stride(int la, int lb, int max_npp);
 
 // S, T (kinetic) or V (attraction to point charges) over all ordered shell pairs
 // of class (la, lb) into out[n][n] (AO order). kind: 0 S, 1 T, 2 V.
@@ -109,17 +144,17 @@ cudaError_t launch_three_center_grad(int la, int lb, const PairTask* tasks, int 
                                      const DevShell* orb, const DevShell* aux, const double* exps,
                                      const double* coefs, const int* const* alist_by_l, const int* count_by_l,
                                      const double* btable, GradWeights g, GradPairData pd, double* gorb,
-                                     double* gaux, cudaStream_t stream);
+                                     double* gaux, Branches& br);
 // Shared memory of one pair's data: max_npp primitive pairs of class (la, lb).
 size_t three_center_grad_smem(int la, int lb, int max_npp);
 // WK: only entries with row <= column are read (its upper triangle).
 cudaError_t launch_metric_grad(const DevShell* aux, const double* exps, const double* coefs,
                                const int* const* aux_by_l, const int* count, const double* btable, const double* WJ,
-                               const double* WK, int64_t ldw, double* gaux, cudaStream_t stream);
+                               const double* WK, int64_t ldw, double* gaux, Branches& br);
 cudaError_t launch_one_electron_grad(int la, int lb, const int2* tasks, int ntasks, const DevShell* orb,
                                      const double* exps, const double* coefs, const double* charges,
                                      const double* positions, int natoms, const double* btable, const double* D,
-                                     const double* W, int64_t n, double* gorb1, double* gatom, cudaStream_t stream);
+                                     const double* W, int64_t n, double* gorb1, double* gatom, Branches& br);
 
 // Exact (ab|cd) over all shell quartets of a small table into out[n][n][n][n].
 cudaError_t launch_four_center(const DevShell* shells, int ns, const double* exps, const double* coefs,

@@ -28,6 +28,7 @@ constexpr int kMaxOrbContr[3] = {3, 2, 1};  // general contractions per l (cc-pV
 constexpr int kBoysTerms = 8;
 // one order more than the integrals need, for their first derivatives
 constexpr int kBoysOrders = 2 * kMaxOrbL + kMaxAuxL + 1 + kBoysTerms;  // 17
+constexpr int kBoysStride = kBoysOrders + 1;  // a grid point's row: the orders and exp(-T)
 constexpr double kBoysStep = 0.05;
 constexpr double kBoysTmax = 36.0;
 constexpr int kBoysGrid = 721;  // T = 0 .. 36 inclusive
@@ -77,27 +78,57 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr double kTwoPi52 = 34.98683665524972;  // 2 pi^(5/2)
 // The matrices live in __constant__ memory of the translation unit that uses them.
 
-// F_0..F_L at T. `table` is [kBoysGrid][kBoysOrders].
+// F_0..F_L at T. `table` is [kBoysGrid][kBoysStride]: F_0 .. F_16 and exp(-T) at each grid point.
+// The serial chain is what bounds it, so it holds no division (the constants' reciprocals fold at
+// compile time; seven divisions of the Taylor sum and L of the recursion were most of a primitive
+// triple's time) and exp(-T) is the grid's value times the Taylor polynomial of exp(T0 - T).
 template <int L>
 __device__ __forceinline__ void boys(double T, const double* __restrict__ table, double* F) {
-    const double et = exp(-T);
     if (T < kBoysTmax) {
         const int j = __double2int_rn(T * (1.0 / kBoysStep));
-        const double d = j * kBoysStep - T;  // T0 - T
-        const double* row = table + j * kBoysOrders + L;
+        const double* row = table + j * kBoysStride;
+        const double d = __dmul_rn((double)j, kBoysStep) - T;  // T0 - T, T0 rounded as the table's
         // F_L(T) = sum_k F_{L+k}(T0) (T0 - T)^k / k!
-        double v = __ldg(row + kBoysTerms - 1);
+        double v = __ldg(row + L + kBoysTerms - 1);
 #pragma unroll
-        for (int k = kBoysTerms - 1; k >= 1; --k) v = __ldg(row + k - 1) + v * d / k;
+        for (int k = kBoysTerms - 1; k >= 1; --k) v = __ldg(row + L + k - 1) + v * (d * (1.0 / k));
         F[L] = v;
+        if constexpr (L > 0) {
+            double e = 1.0;
 #pragma unroll
-        for (int n = L; n >= 1; --n) F[n - 1] = (2.0 * T * F[n] + et) / (2 * n - 1);
+            for (int k = kBoysTerms - 1; k >= 1; --k) e = 1.0 + e * (d * (1.0 / k));
+            e *= __ldg(row + kBoysOrders);
+#pragma unroll
+            for (int n = L; n >= 1; --n)
+                F[n - 1] = F[n] * (2.0 * T * (1.0 / (2 * n - 1))) + e * (1.0 / (2 * n - 1));
+        }
     } else {
-        F[0] = 0.5 * sqrt(3.14159265358979323846 / T);
         const double inv2T = 0.5 / T;
+        F[0] = sqrt(0.5 * kPi * inv2T);  // sqrt(pi / T) / 2
+        if constexpr (L > 0) {
+            const double e = exp(-T);
 #pragma unroll
-        for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - et) * inv2T;
+            for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - e) * inv2T;
+        }
     }
+}
+
+// 1 / (p + q) and 1 / sqrt(p + q) from one reciprocal square root: its square, corrected by one
+// Newton step (the step's residual is one fused operation), is as good as a division.
+__device__ __forceinline__ void inverse_sum(double p, double q, double& inv, double& inv_sqrt) {
+    const double s = p + q;
+    inv_sqrt = rsqrt(s);
+    inv = inv_sqrt * inv_sqrt;
+    inv = fma(inv, fma(-s, inv, 1.0), inv);
+}
+
+// (2q)^-L from 1 / q.
+template <int L>
+__device__ __forceinline__ double half_power(double inv_q) {
+    double v = 1.0;
+#pragma unroll
+    for (int k = 0; k < L; ++k) v *= 0.5 * inv_q;
+    return v;
 }
 
 // R^0_tuv(alpha, X, Y, Z) for t+u+v <= L into R[tet(t,u,v)]. Up to L = 4 the
