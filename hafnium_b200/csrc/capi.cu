@@ -919,14 +919,22 @@ int hf_dims(const hf_ctx* ctx, int64_t* n_ao, int64_t* n_aux) {
 static int build_metric(hf_ctx* ctx) {
     const size_t bytes = sizeof(double) * (size_t)ctx->naux * ctx->naux;
     if (!ctx->d_metric && alloc(ctx, (void**)&ctx->d_metric, bytes)) return HF_ERR_OOM;
+    double* scaled = nullptr;
+    if (talloc(ctx, (void**)&scaled, sizeof(double) * ctx->h_coefs.size())) return HF_ERR_OOM;
     {
         BranchLoan loan(ctx);
-        HF_CU(loan.br.fork());
-        HF_CU(launch_metric(ctx->d_aux, ctx->d_exps, ctx->d_coefs, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable,
-                            ctx->d_metric, ctx->naux, loan.br));
-        HF_CU(loan.br.join());
+        cudaError_t e = launch_scale_primitives(ctx->d_aux, (int)ctx->aux.size(), ctx->d_exps, ctx->d_coefs, scaled,
+                                                ctx->stream);
+        if (e == cudaSuccess) e = loan.br.fork();
+        if (e == cudaSuccess)
+            e = launch_metric(ctx->d_aux, ctx->d_exps, scaled, ctx->d_aux_by_l, ctx->aux_count, ctx->d_btable,
+                              ctx->d_metric, ctx->naux, loan.br);
+        const cudaError_t je = loan.br.join();
+        trelease(ctx, scaled);
+        HF_CU(e);
+        HF_CU(je);
     }
-    ctx->stats.kernel_launches += 25;
+    ctx->stats.kernel_launches += 26;
     return check_async(ctx, "metric");
 }
 
@@ -2130,7 +2138,9 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
     cudaMemGetInfo(&freeb, &totalb);
     const size_t per_p = sizeof(double) * (nn + (size_t)n * o);
     const size_t budget = std::min<size_t>((size_t)8 << 30, freeb / 3);
-    const int64_t pb_max = std::max<int64_t>(16, (int64_t)(budget / per_p));
+    // a block of the auxiliary functions, never more than there are (8 GB of weights for 904 of them
+    // took 3 ms to map per call)
+    const int64_t pb_max = std::min<int64_t>(N, std::max<int64_t>(16, (int64_t)(budget / per_p)));
     double* Zt = tmp.take((size_t)n * o * (pb_max + 8));
     double* GK = tmp.take(nn * (pb_max + 8));
     if (!Zt || !GK) return fail(ctx, HF_ERR_OOM, "no room for the exchange weights of a block");

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
                                                            const double* __restrict__ btable, GradWeights g,
                                                            const int64_t* __restrict__ offsets,
                                                            const double* __restrict__ pdata,
-                                                           const int* __restrict__ npps,
+                                                           const int* __restrict__ npps, int share,
                                                            double* __restrict__ gorb, double* __restrict__ gaux) {
     using PL = GradPairLayout<LA, LB>;
     using SH = GradCenterShape<LA, LB, LP>;
@@ -300,8 +300,11 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wslot = lane / NSP, mp = lane - wslot * NSP;
     const int slot = warp * SPW + wslot;
-    const int ia = blockIdx.y * SH::SPB + slot;
-    const bool active = wslot < SPW && ia < nalist;
+    // `share` slots of a warp take the triples of one shell in turn (their sums are added at the end)
+    const int spw = SPW / share, part = wslot % share;
+    const int ia = (blockIdx.y * (kGradCenterThreads / 32) + warp) * spw + wslot / share;
+    const bool active = wslot < spw * share && ia < nalist;
+    const int step = TPR * share;
     const double fac = task.first == task.second ? 1.0 : 2.0;
     // per-thread sums for the two orbital centres: A_J[3] A_K[3] B_J[3] B_K[3]
     // (J parts with the factor c_P applied)
@@ -345,15 +348,15 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
 #pragma unroll
             for (int m = 0; m < PL::NSAB; ++m) gk[k][m] = 0.0;
     }
-    // rounds of this warp: its slowest shell's triples over TPR
-    const int rounds = __reduce_max_sync(0xffffffffu, (ntrip + TPR - 1) / TPR);
+    // rounds of this warp: its slowest shell's triples over TPR and its slots
+    const int rounds = __reduce_max_sync(0xffffffffu, (ntrip + step - 1) / step);
     const int nnz = s_nnz[active ? mp : 0];
     const int* __restrict__ nzc = s_nzc + (active ? mp : 0) * NCP;
     const double* __restrict__ nzw = s_nzw + (active ? mp : 0) * NCP;
 
-    // this thread's triple t = r TPR + mp as (auxiliary primitive i, primitive pair pp),
-    // advanced by TPR per round; the auxiliary primitive's factors are kept while i stays
-    int ti = mp / npp, tpp = mp - (mp / npp) * npp;
+    // this thread's triple t = r step + part TPR + mp as (auxiliary primitive i, primitive pair pp),
+    // advanced by step per round; the auxiliary primitive's factors are kept while i stays
+    int ti = (part * TPR + mp) / npp, tpp = (part * TPR + mp) - ti * npp;
     int ci = -1;
     double q = 0.0, cq = 0.0;
     for (int r = 0; r < rounds; ++r) {
@@ -385,7 +388,7 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
                 }
                 // 2 pi^(5/2) / (p q sqrt(p + q)) c_P (2q)^-l_P (-1)^l_P
                 row[NR] = inv_root * s[PL::INV] * cq;
-                tpp += TPR;
+                tpp += step;
                 while (tpp >= npp) {
                     tpp -= npp;
                     ++ti;
@@ -459,7 +462,10 @@ __global__ void __launch_bounds__(kGradCenterThreads) k_three_center_grad(const 
         }
         __syncwarp();
     }
-    if (active) {
+    for (int o = share >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 12; ++k) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o * NSP);
+    if (active && part == 0) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             atomicAdd(gaux + (int64_t)pshell * 6 + d, fac * cP * acc[d]);
@@ -487,7 +493,6 @@ static cudaError_t three_center_grad_one(const PairTask* tasks, int ntasks, int 
                                          GradPairData pd, double* gorb, double* gaux, cudaStream_t stream) {
     if (ntasks == 0 || nalist == 0) return cudaSuccess;
     using SH = GradCenterShape<LA, LB, LP>;
-    (void)max_npp;  // the pair data is read from global memory
     const size_t smem = sizeof(double) * (size_t)SH::R_DOUBLES;
     // the attribute covers the dynamic part; the static tables count against
     // the 48 KB default too
@@ -496,9 +501,11 @@ static cudaError_t three_center_grad_one(const PairTask* tasks, int ntasks, int 
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    dim3 grid(ntasks, (nalist + SH::SPB - 1) / SH::SPB);
+    const int share = triple_share(ntasks, nalist, SH::SPW, kGradCenterThreads / 32, max_npp, SH::TPR, INT32_MAX);
+    const int per_cta = kGradCenterThreads / 32 * (SH::SPW / share);
+    dim3 grid(ntasks, (nalist + per_cta - 1) / per_cta);
     k_three_center_grad<LA, LB, LP><<<grid, kGradCenterThreads, smem, stream>>>(
-        tasks, orb, aux, exps, coefs, alist, nalist, btable, g, pd.offsets, pd.data, pd.npps, gorb, gaux);
+        tasks, orb, aux, exps, coefs, alist, nalist, btable, g, pd.offsets, pd.data, pd.npps, share, gorb, gaux);
     return cudaGetLastError();
 }
 

@@ -120,7 +120,7 @@ std::vector<double> boys_grid_host() {
     static std::vector<double> cached;
     std::lock_guard<std::mutex> lock(mutex);
     if (!cached.empty()) return cached;
-    std::vector<double> g(kBoysGrid * kBoysStride);
+    std::vector<double> g(kBoysGrid * kBoysOrders);
     const int nmax = kBoysOrders - 1;
     for (int j = 0; j < kBoysGrid; ++j) {
         const double t = j * kBoysStep;
@@ -131,9 +131,8 @@ std::vector<double> boys_grid_host() {
             sum += term;
             if (term < sum * 1e-17) break;
         }
-        double* row = &g[j * kBoysStride];
+        double* row = &g[j * kBoysOrders];
         row[nmax] = et * sum;
-        row[kBoysOrders] = et;
         for (int n = nmax; n >= 1; --n) row[n - 1] = (2.0 * t * row[n] + et) / (2 * n - 1);
     }
     cached = g;
@@ -179,9 +178,38 @@ cudaError_t launch_boys_values(const double* t, int64_t count, int n_max, const 
 static_assert(kBoysOrders - kBoysTerms == 9, "launch_boys_values covers orders 0..9");
 
 // ------------------------------------------------------------- (P|Q) metric
+// scaled[i] = c_i (2 a_i)^-l for every auxiliary primitive: taken once per primitive, a power per
+// primitive pair and component was a large part of the metric's time.
+__global__ void k_scale_primitives(const DevShell* __restrict__ aux, int naux_shells, const double* __restrict__ exps,
+                                   const double* __restrict__ coefs, double* __restrict__ scaled) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= naux_shells) return;
+    const DevShell P = aux[s];
+    for (int i = 0; i < P.nprim; ++i) {
+        const double c = coefs[P.coef + i], a = exps[P.prim + i];
+        double v = c;
+        switch (P.l) {  // constant exponents
+            case 0: v = c * pow(2.0 * a, -(double)0); break;
+            case 1: v = c * pow(2.0 * a, -(double)1); break;
+            case 2: v = c * pow(2.0 * a, -(double)2); break;
+            case 3: v = c * pow(2.0 * a, -(double)3); break;
+            case 4: v = c * pow(2.0 * a, -(double)4); break;
+        }
+        scaled[P.coef + i] = v;
+    }
+}
+static_assert(kMaxAuxL == 4, "k_scale_primitives covers l = 0..4");
+
+cudaError_t launch_scale_primitives(const DevShell* aux, int shells, const double* exps, const double* coefs,
+                                    double* scaled, cudaStream_t stream) {
+    if (shells < 1) return cudaSuccess;
+    k_scale_primitives<<<(shells + 63) / 64, 64, 0, stream>>>(aux, shells, exps, coefs, scaled);
+    return cudaGetLastError();
+}
+
 template <int LP, int LQ>
 __global__ void __launch_bounds__(128) k_metric(const DevShell* __restrict__ aux, const double* __restrict__ exps,
-                                                const double* __restrict__ coefs, const int* __restrict__ plist,
+                                                const double* __restrict__ scaled, const int* __restrict__ plist,
                                                 int np, const int* __restrict__ qlist, int nq,
                                                 const double* __restrict__ btable, double* __restrict__ M,
                                                 int64_t ldm) {
@@ -204,18 +232,15 @@ __global__ void __launch_bounds__(128) k_metric(const DevShell* __restrict__ aux
     const double X = P.x - Q.x, Y = P.y - Q.y, Z = P.z - Q.z;
     for (int i = 0; i < P.nprim; ++i) {
         const double p = exps[P.prim + i];
-        const double inv_p = 1.0 / p;
-        const double cp = coefs[P.coef + i] * half_power<LP>(inv_p) * kTwoPi52 * inv_p;
+        const double cp = scaled[P.coef + i];
         for (int j = 0; j < Q.nprim; ++j) {
             const double q = exps[Q.prim + j];
-            const double inv_q = 1.0 / q;
-            double cq = coefs[Q.coef + j] * half_power<LQ>(inv_q) * inv_q;
+            double cq = scaled[Q.coef + j];
             if (LQ & 1) cq = -cq;
-            double inv_pq, inv_root;
-            inverse_sum(p, q, inv_pq, inv_root);
+            const double alpha = p * q / (p + q);
             double R[ntet(L)];
-            hermite_r<L>(p * q * inv_pq, X, Y, Z, btable, R);
-            const double pref = inv_root * cp * cq;  // 2 pi^(5/2) / (p q sqrt(p + q)) and the coefficients
+            hermite_r<L>(alpha, X, Y, Z, btable, R);
+            const double pref = kTwoPi52 / (p * q * sqrt(p + q)) * cp * cq;
             double h[NCQ];
 #pragma unroll
             for (int b = 0; b < NCQ; ++b) {
@@ -469,7 +494,7 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
                                                       const int* __restrict__ alist, int nalist,
                                                       const double* __restrict__ btable, ChunkDesc chunk,
                                                       const double* __restrict__ pdata, int64_t pstride,
-                                                      const int* __restrict__ npps, int r_offset,
+                                                      const int* __restrict__ npps, int r_offset, int share,
                                                       double* __restrict__ T) {
     using PL = PairLayout<LA, LB>;
     using SH = ThreeCenterShape<LA, LB, LP>;
@@ -510,18 +535,21 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
     const DevShell B = orb[task.swap ? task.first : task.second];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // `share` slots of a warp take the triples of one shell in turn (their sums are added at the end)
     const int wslot = lane / NSP, mp = lane - wslot * NSP;
     const int slot = warp * SPW + wslot;
-    const int ia = blockIdx.y * SH::SPB + slot;
-    const bool active = wslot < SPW && ia < nalist;
+    const int spw = SPW / share, part = wslot % share;
+    const int ia = (blockIdx.y * 4 + warp) * spw + wslot / share;
+    const bool active = wslot < spw * share && ia < nalist;
+    const int step = TPR * share;
     DevShell P{};
     int ntrip = 0;
     if (active) {
         P = aux[alist[ia]];
         ntrip = P.nprim * npp;
     }
-    // rounds of this warp: its slowest shell's triples over TPR
-    const int rounds = __reduce_max_sync(0xffffffffu, (ntrip + TPR - 1) / TPR);
+    // rounds of this warp: its slowest shell's triples over TPR and its slots
+    const int rounds = __reduce_max_sync(0xffffffffu, (ntrip + step - 1) / step);
     const int nnz = s_nnz[active ? mp : 0];
 
     double acc[PL::KK][PL::NSAB];
@@ -530,9 +558,9 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
 #pragma unroll
         for (int m = 0; m < PL::NSAB; ++m) acc[k][m] = 0.0;
 
-    // this thread's triple t = r TPR + mp as (auxiliary primitive i, primitive pair pp),
-    // advanced by TPR per round; the auxiliary primitive's factors are kept while i stays
-    int ti = mp / npp, tpp = mp - (mp / npp) * npp;
+    // this thread's triple t = r step + part TPR + mp as (auxiliary primitive i, primitive pair pp),
+    // advanced by step per round; the auxiliary primitive's factors are kept while i stays
+    int ti = (part * TPR + mp) / npp, tpp = (part * TPR + mp) - ti * npp;
     int ci = -1;
     double q = 0.0, cq = 0.0;
     for (int r = 0; r < rounds; ++r) {
@@ -553,11 +581,11 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
             }
             const double* s = smem + pp * PL::STRIDE;
             const double p = s[0];
-            // the reduced exponent and the prefactor 2 pi^(5/2) / (p q sqrt(p+q))
-            double inv_pq, inv_root;
-            inverse_sum(p, q, inv_pq, inv_root);
+            // one division per primitive triple: 1/(p+q) gives both the reduced
+            // exponent and the prefactor 2 pi^(5/2) / (p q sqrt(p+q))
+            const double inv_pq = 1.0 / (p + q);
             const double alpha = p * q * inv_pq;
-            const double pref = s[4] * inv_root * cq;
+            const double pref = s[4] * sqrt(inv_pq) * cq;
             if constexpr (NSP == 1) {
                 hermite_r<L>(alpha, s[1] - P.x, s[2] - P.y, s[3] - P.z, btable, R);
                 const double scale = pref * c_c2s[c2s_offset(LP)];  // the single weight of l_P = 0
@@ -575,7 +603,7 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
                 }
                 row[NR] = pref;
             }
-            tpp += TPR;
+            tpp += step;
             while (tpp >= npp) {
                 tpp -= npp;
                 ++ti;
@@ -632,7 +660,12 @@ __global__ void __launch_bounds__(128) k_three_center(const PairTask* __restrict
             __syncwarp();
         }
     }
-    if (!active) return;
+    for (int o = share >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < PL::KK; ++k)
+#pragma unroll
+            for (int m = 0; m < PL::NSAB; ++m) acc[k][m] += __shfl_down_sync(0xffffffffu, acc[k][m], o * NSP);
+    if (!active || part != 0) return;
 
     // Scatter into the chunk: element (mu, nu) in AO order, both orders where the
     // tile is on or above the diagonal and its row belongs to this chunk.
@@ -686,9 +719,11 @@ static cudaError_t three_center_one(const PairTask* tasks, int ntasks, int max_n
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    dim3 grid(ntasks, (nalist + SH::SPB - 1) / SH::SPB);  // 4 warps of SPW shells
+    const int share = triple_share(ntasks, nalist, SH::SPW, 4, max_npp, SH::TPR, kShareTasks);
+    const int per_cta = 4 * (SH::SPW / share);
+    dim3 grid(ntasks, (nalist + per_cta - 1) / per_cta);  // 4 warps of SPW / share shells
     k_three_center<LA, LB, LP><<<grid, 128, smem, stream>>>(tasks, orb, aux, exps, coefs, alist, nalist, btable,
-                                                            chunk, pd.data, pd.stride, pd.npps, r_offset, T);
+                                                            chunk, pd.data, pd.stride, pd.npps, r_offset, share, T);
     return cudaGetLastError();
 }
 
@@ -714,6 +749,8 @@ cudaError_t launch_three_center(int la, int lb, const PairTask* tasks, int ntask
 }
 
 // ---------------------------------------------------------- S, T and V
+// The order and the contraction of these sums are kept as they are: the orbitals of a first density
+// amplify another rounding of h, which a wider split over the primitive pairs changed in V.
 template <int LA, int LB, int KIND>
 __global__ void __launch_bounds__(128) k_one_electron(const int2* __restrict__ tasks, int ntasks,
                                                       const DevShell* __restrict__ orb,
@@ -759,7 +796,7 @@ __global__ void __launch_bounds__(128) k_one_electron(const int2* __restrict__ t
                 for (int h = 0; h < ntet(LAB); ++h) Rs[h] = 0.0;
                 for (int c = lane; c < natoms; c += LANES) {
                     double R[ntet(LAB)];
-                    hermite_r<LAB>(p, px - positions[3 * c], py - positions[3 * c + 1], pz - positions[3 * c + 2],
+                    hermite_r<LAB, true>(p, px - positions[3 * c], py - positions[3 * c + 1], pz - positions[3 * c + 2],
                                    btable, R);
                     const double z = charges[c];
 #pragma unroll
@@ -789,7 +826,7 @@ __global__ void __launch_bounds__(128) k_one_electron(const int2* __restrict__ t
                         cart[ca][cb] = pref * s;
                     }
             } else {
-                const double ov = kPi / p * sqrt(kPi / p);
+                const double ov = pow(kPi / p, 1.5);
 #pragma unroll
                 for (int ca = 0; ca < NCA; ++ca)
 #pragma unroll

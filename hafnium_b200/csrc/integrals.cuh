@@ -16,6 +16,24 @@ struct DevShell {
     int l, nprim, ncontr, prim, coef, fn;
 };
 
+// Slots of a warp (1, 2, 4 .. spw) that share one auxiliary shell's primitive triples in the
+// three-centre kernels. A small molecule's classes have too few (pair, shell) tasks for the chip and a
+// slot's triples are one serial chain (up to 81 primitive pairs times the auxiliary shell's
+// primitives), so slots are shared while there are at most two CTAs an SM and the chain is longer
+// than the slots; a large molecule keeps a slot per shell. Sharing changes the order of a triple sum,
+// which the fit amplifies by the metric's condition, so (P|uv) does it only for classes of up to
+// kShareTasks pairs; the derivatives are not behind a fit. (H2O)2: (P|uv) 0.49 -> 0.29 ms.
+constexpr int kShareTasks = 64;
+inline int triple_share(int ntasks, int nalist, int spw, int warps, int max_npp, int tpr, int most_tasks) {
+    int share = 1;
+    while (ntasks <= most_tasks && 2 * share <= spw && 2 * share * tpr <= max_npp) {
+        const int per_cta = warps * (spw / (2 * share));
+        if ((int64_t)ntasks * ((nalist + per_cta - 1) / per_cta) > 2 * 148) break;
+        share *= 2;
+    }
+    return share;
+}
+
 // The part of the packed fitted tensor a three-centre launch fills: tile rows
 // [row0, row1) of the upper triangle of 64x64 (mu, nu) tiles, laid out as
 // T[col][q] with col = (tile - tile_base) * 4096 + (mu % 64) * 64 + nu % 64.
@@ -90,7 +108,12 @@ constexpr int kBoysMaxOrder = kBoysOrders - kBoysTerms;
 cudaError_t launch_boys_values(const double* t, int64_t count, int n_max, const double* btable, double* out,
                                cudaStream_t stream);
 
-// (P|Q) for all aux shells into M[N][N] (internal order, row-major, ld = ldm).
+// scaled[i] = coefs[i] (2 exps[i])^-l over the auxiliary primitives, at the shells' coefficient offsets.
+cudaError_t launch_scale_primitives(const DevShell* aux, int shells, const double* exps, const double* coefs,
+                                    double* scaled, cudaStream_t stream);
+
+// (P|Q) for all aux shells into M[N][N] (internal order, row-major, ld = ldm); coefs:
+// those of launch_scale_primitives.
 cudaError_t launch_metric(const DevShell* aux, const double* exps, const double* coefs,
                           const int* const* aux_by_l_dev, const int* aux_count, const double* btable,
                           double* M, int64_t ldm, Branches& br);

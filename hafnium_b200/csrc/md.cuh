@@ -28,7 +28,6 @@ constexpr int kMaxOrbContr[3] = {3, 2, 1};  // general contractions per l (cc-pV
 constexpr int kBoysTerms = 8;
 // one order more than the integrals need, for their first derivatives
 constexpr int kBoysOrders = 2 * kMaxOrbL + kMaxAuxL + 1 + kBoysTerms;  // 17
-constexpr int kBoysStride = kBoysOrders + 1;  // a grid point's row: the orders and exp(-T)
 constexpr double kBoysStep = 0.05;
 constexpr double kBoysTmax = 36.0;
 constexpr int kBoysGrid = 721;  // T = 0 .. 36 inclusive
@@ -78,43 +77,82 @@ constexpr double kPi = 3.14159265358979323846;
 constexpr double kTwoPi52 = 34.98683665524972;  // 2 pi^(5/2)
 // The matrices live in __constant__ memory of the translation unit that uses them.
 
-// F_0..F_L at T. `table` is [kBoysGrid][kBoysStride]: F_0 .. F_16 and exp(-T) at each grid point.
-// The serial chain is what bounds it, so it holds no division (the constants' reciprocals fold at
-// compile time; seven divisions of the Taylor sum and L of the recursion were most of a primitive
-// triple's time) and exp(-T) is the grid's value times the Taylor polynomial of exp(T0 - T).
-template <int L>
+// x / D, correctly rounded, by a multiplication with the rounded reciprocal and one correction
+// (Markstein, IBM J. Res. Dev. 34, 111 (1990)): the residual x - q D of the first quotient is exact in
+// one fused operation.
+template <int D>
+__device__ __forceinline__ double divide_by(double x) {
+    if constexpr ((D & (D - 1)) == 0) {
+        return x * (1.0 / D);
+    } else {
+        constexpr double r = 1.0 / D;
+        const double q = __dmul_rn(x, r);
+        return __fma_rn(__fma_rn(-q, (double)D, x), r, q);
+    }
+}
+// The same with a divisor known at run time and its rounded reciprocal r = 1 / d.
+__device__ __forceinline__ double divide_by(double x, double d, double r) {
+    const double q = __dmul_rn(x, r);
+    return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
+template <int N>
+struct BoysSteps {
+    // v <- c_(N-1) + v d / N, N = from .. 1
+    static __device__ __forceinline__ double taylor(const double* __restrict__ row, double v, double d) {
+        if constexpr (N == 0) {
+            return v;
+        } else {
+            const double c = __ldg(row + N - 1);
+            const double w = N == 1 ? __fma_rn(v, d, c) : __dadd_rn(c, divide_by<N>(__dmul_rn(v, d)));
+            return BoysSteps<N - 1>::taylor(row, w, d);
+        }
+    }
+    // F[n - 1] = (2 T F[n] + e^-T) / (2 n - 1), n = N .. 1
+    static __device__ __forceinline__ void down(double* F, double two_t, double et) {
+        if constexpr (N > 0) {
+            F[N - 1] = divide_by<2 * N - 1>(__fma_rn(two_t, F[N], et));
+            BoysSteps<N - 1>::down(F, two_t, et);
+        }
+    }
+};
+
+// F_0..F_L at T. `table` is [kBoysGrid][kBoysOrders]. The serial chain is what bounds it: its
+// divisions by constants are three operations each with the same rounding as a division (as divisions,
+// seven in the Taylor sum and L in the recursion were most of a primitive triple's time). The metric's
+// condition amplifies an ulp here to 1e-12 in J, so the values stay what they were, bit for bit.
+// DIVIDE keeps the divisions in the source: with alpha r^2 inlined, the nuclear attraction's T is
+// contracted into what surrounds it, and only the same source gave the same h.
+template <int L, bool DIVIDE = false>
 __device__ __forceinline__ void boys(double T, const double* __restrict__ table, double* F) {
+    const double et = exp(-T);
     if (T < kBoysTmax) {
         const int j = __double2int_rn(T * (1.0 / kBoysStep));
-        const double* row = table + j * kBoysStride;
-        const double d = __dmul_rn((double)j, kBoysStep) - T;  // T0 - T, T0 rounded as the table's
+        const double d = j * kBoysStep - T;  // T0 - T
+        const double* row = table + j * kBoysOrders + L;
         // F_L(T) = sum_k F_{L+k}(T0) (T0 - T)^k / k!
-        double v = __ldg(row + L + kBoysTerms - 1);
+        if constexpr (DIVIDE) {
+            double v = __ldg(row + kBoysTerms - 1);
 #pragma unroll
-        for (int k = kBoysTerms - 1; k >= 1; --k) v = __ldg(row + L + k - 1) + v * (d * (1.0 / k));
-        F[L] = v;
-        if constexpr (L > 0) {
-            double e = 1.0;
+            for (int k = kBoysTerms - 1; k >= 1; --k) v = __ldg(row + k - 1) + v * d / k;
+            F[L] = v;
 #pragma unroll
-            for (int k = kBoysTerms - 1; k >= 1; --k) e = 1.0 + e * (d * (1.0 / k));
-            e *= __ldg(row + kBoysOrders);
-#pragma unroll
-            for (int n = L; n >= 1; --n)
-                F[n - 1] = F[n] * (2.0 * T * (1.0 / (2 * n - 1))) + e * (1.0 / (2 * n - 1));
+            for (int n = L; n >= 1; --n) F[n - 1] = (2.0 * T * F[n] + et) / (2 * n - 1);
+        } else {
+            F[L] = BoysSteps<kBoysTerms - 1>::taylor(row, __ldg(row + kBoysTerms - 1), d);
+            BoysSteps<L>::down(F, 2.0 * T, et);
         }
     } else {
+        F[0] = 0.5 * sqrt(3.14159265358979323846 / T);
         const double inv2T = 0.5 / T;
-        F[0] = sqrt(0.5 * kPi * inv2T);  // sqrt(pi / T) / 2
-        if constexpr (L > 0) {
-            const double e = exp(-T);
 #pragma unroll
-            for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - e) * inv2T;
-        }
+        for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - et) * inv2T;
     }
 }
 
 // 1 / (p + q) and 1 / sqrt(p + q) from one reciprocal square root: its square, corrected by one
-// Newton step (the step's residual is one fused operation), is as good as a division.
+// Newton step (the step's residual is one fused operation), is as good as a division (the derivative
+// kernels; the integrals behind the fit keep their division's and root's exact rounding).
 __device__ __forceinline__ void inverse_sum(double p, double q, double& inv, double& inv_sqrt) {
     const double s = p + q;
     inv_sqrt = rsqrt(s);
@@ -135,11 +173,11 @@ __device__ __forceinline__ double half_power(double inv_q) {
 // recursion is unrolled so the table stays in registers; above, the loops are
 // left rolled (the table lives in L1-resident local memory), which keeps the
 // kernels compact and their compile time short.
-template <int L>
+template <int L, bool DIVIDE = false>
 __device__ __forceinline__ void hermite_r(double alpha, double X, double Y, double Z,
                                           const double* __restrict__ btable, double* R) {
     double F[L + 1];
-    boys<L>(alpha * (X * X + Y * Y + Z * Z), btable, F);
+    boys<L, DIVIDE>(alpha * (X * X + Y * Y + Z * Z), btable, F);
     const double m2a = -2.0 * alpha;
     double pw[L + 1];
     pw[0] = 1.0;
