@@ -798,13 +798,9 @@ int hf_batch_load(hf_batch* b, const double* overlap, const double* core, const 
     std::vector<double> big(b->count, 1e300);
     HB_CU(cudaMemcpyAsync(d_piv, big.data(), sizeof(double) * b->count, cudaMemcpyHostToDevice, s));
     HB_CU(cudaMemsetAsync(d_info, 0, sizeof(int) * 2 * b->count, s));
-    for (int c = 0; c < b->count; ++c) {
-        double* L = b->T1 + (int64_t)c * b->nn;
-        HB_CU(cholesky_lower(L, (int)b->n, b->n, d_info + c, d_piv + c, s));
-        // XT = L^-1 (row-major lower), X = its transpose; the K chunk buffer (>= n x 64) as work
-        HB_CU(triangular_inverse(L, (int)b->n, b->n, b->XT + (int64_t)c * b->nn, b->X + (int64_t)c * b->nn, b->Xch,
-                                 s));
-    }
+    // XT = L^-1 (row-major lower), X = its transpose; work: the K chunk buffer (>= n x 64 per cluster)
+    HB_CU(cholesky_lower(b->T1, (int)b->n, b->n, d_info, d_piv, b->Xch, s, b->count, b->nn));
+    HB_CU(triangular_inverse(b->T1, (int)b->n, b->n, b->XT, b->X, b->Xch, s, b->count, b->nn, b->npad * 64));
     k_frobenius2<<<b->count, kThreads, 0, s>>>(b->X, b->nn, b->T2);
     HB_CU(cudaGetLastError());
     std::vector<int> info(b->count);

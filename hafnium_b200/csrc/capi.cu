@@ -1076,7 +1076,7 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
     double *L = nullptr, *Linv = nullptr, *LinvT = nullptr, *wk = nullptr;
     const size_t nn = (size_t)N * N;
     if (talloc(ctx, (void**)&L, nn * 8) || talloc(ctx, (void**)&Linv, nn * 8) || talloc(ctx, (void**)&LinvT, nn * 8) ||
-        talloc(ctx, (void**)&wk, (size_t)N * 64 * 8)) {
+        talloc(ctx, (void**)&wk, 8 * std::max(cholesky_work_doubles(N), inverse_work_doubles(N)))) {
         trelease(ctx, L);
         trelease(ctx, Linv);
         trelease(ctx, LinvT);
@@ -1087,11 +1087,12 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
     HF_CU(cudaMemsetAsync(ctx->d_info, 0, sizeof(int), ctx->stream));
     const double big = 1e300;
     HF_CU(cudaMemcpyAsync(ctx->d_scalar, &big, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    HF_CU(cholesky_lower(L, N, N, ctx->d_info, ctx->d_scalar, ctx->stream));
+    HF_CU(cholesky_lower(L, N, N, ctx->d_info, ctx->d_scalar, wk, ctx->stream));
+    HF_CU(max_diagonal(ctx->d_metric, N, N, ctx->d_scalar + 1, ctx->stream));
     int info = 0;
-    double pivmin = 0.0;
+    double pivot[2] = {0.0, 0.0};  // the smallest pivot's root, the largest diagonal element
     HF_CU(cudaMemcpyAsync(&info, ctx->d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    HF_CU(cudaMemcpyAsync(&pivmin, ctx->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    HF_CU(cudaMemcpyAsync(pivot, ctx->d_scalar, sizeof(pivot), cudaMemcpyDeviceToHost, ctx->stream));
     HF_CU(cudaStreamSynchronize(ctx->stream));
     if (info != 0) {
         trelease(ctx, L);
@@ -1101,13 +1102,7 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
         return fail(ctx, HF_ERR_NUMERIC, "the Coulomb metric is not positive definite (pivot " + std::to_string(info - 1) +
                                              ")");
     }
-    {
-        std::vector<double> diag(N);
-        HF_CU(cudaMemcpy2D(diag.data(), sizeof(double), ctx->d_metric, sizeof(double) * ((size_t)N + 1), sizeof(double),
-                           N, cudaMemcpyDeviceToHost));
-        const double dmax = *std::max_element(diag.begin(), diag.end());
-        ctx->stats.min_pivot_ratio = pivmin * pivmin / dmax;
-    }
+    ctx->stats.min_pivot_ratio = pivot[0] * pivot[0] / pivot[1];
     HF_CU(triangular_inverse(L, N, N, Linv, LinvT, wk, ctx->stream));
     if ((s = check_async(ctx, "inverse factor")) != HF_OK) return s;
     ctx->stats.ms_factor = time_end(ctx);
@@ -2010,7 +2005,7 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
     double* L = tmp.take(NN);
     double* Linv = tmp.take(NN);
     double* LinvT = tmp.take(NN);
-    double* wk = tmp.take((size_t)N * 64);
+    double* wk = tmp.take(std::max(cholesky_work_doubles((int)N), inverse_work_doubles((int)N)));
     double* Gt = tmp.take((size_t)oo * N);
     double* G = tmp.take((size_t)oo * N);
     double* WJ = tmp.take(NN);
@@ -2057,7 +2052,7 @@ int hf_nuclear_gradient(hf_ctx* ctx, const double* C, int64_t nocc, const double
     HF_CU(cudaMemsetAsync(ctx->d_info, 0, sizeof(int), ctx->stream));
     const double big = 1e300;
     HF_CU(cudaMemcpyAsync(ctx->d_scalar, &big, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    HF_CU(cholesky_lower(L, N, N, ctx->d_info, ctx->d_scalar, ctx->stream));
+    HF_CU(cholesky_lower(L, N, N, ctx->d_info, ctx->d_scalar, wk, ctx->stream));
     int info = 0;
     HF_CU(cudaMemcpyAsync(&info, ctx->d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     HF_CU(cudaStreamSynchronize(ctx->stream));

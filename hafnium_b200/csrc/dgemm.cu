@@ -100,6 +100,10 @@ __global__ void __launch_bounds__(threads_of<BM, BN>(), (min_ctas_of<BM, BN, BK,
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gq = lane >> 2, tq = lane & 3;
     const int wm = (warp / WARPS_N) * 32, wn = (warp % WARPS_N) * 32;
+    // a warp whose 32 x 32 outputs lie outside C, or wholly in the triangle that epi leaves out of
+    // its diagonal tiles, only loads: its share of the FP64 pipe goes to the others
+    const bool live = m0 + wm < g.M && n0 + wn < g.N && !(g.epi == 2 && n0 + wn > m0 + wm + 31) &&
+                      !(g.epi == 3 && m0 + wm > n0 + wn + 31);
 
     auto load = [&](int stage, int k0) {
         double* as = As + stage * BM * LD;
@@ -159,6 +163,7 @@ __global__ void __launch_bounds__(threads_of<BM, BN>(), (min_ctas_of<BM, BN, BK,
         asm volatile("cp.async.commit_group;\n" ::);
         const double* as = As + (it % STAGES) * BM * LD;
         const double* bs = Bs + (it % STAGES) * BN * LD;
+        if (!live) continue;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 8) {
             double af[2][4], bf[4][2];
@@ -183,6 +188,7 @@ __global__ void __launch_bounds__(threads_of<BM, BN>(), (min_ctas_of<BM, BN, BK,
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::);
+    if (!live) return;
 
 #pragma unroll
     for (int i = 0; i < 2; ++i)

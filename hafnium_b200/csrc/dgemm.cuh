@@ -14,8 +14,9 @@
 //      row of the full triangle that A's first row is)
 // epi selects the store:
 //   0: C[m][n] (row stride ldc)      1: C[n][m] (transposed store)
-//   2: as 0, only tiles touching the lower triangle (n0 <= m0 + BM - 1)
-//   3: as 0, only tiles touching the upper triangle (m0 <= n0 + BN - 1)
+//   2: as 0, the lower triangle: only CTA tiles, and within them warp tiles of 32 x 32,
+//      that touch it (n0 <= m0 + BM - 1)
+//   3: as 0, the upper triangle in the same way (m0 <= n0 + BN - 1)
 //
 // Batching runs over blockIdx.z with per-batch pointer strides. Optional
 // per-batch arrays: `active` (a batch whose entry is 0 is skipped and its C is
