@@ -556,7 +556,7 @@ cudaError_t gemm(const hf_batch* b, const GemmArgs& g, cudaStream_t s) { return 
 // The Fock build of the clusters in `active`: K from a rank-<= maxr pivoted
 // Cholesky factor of D, J from 2 D, then F and the energy.
 cudaError_t fock_build(hf_batch* b, cudaStream_t s, const int* active, int maxr) {
-    const int opad = (int)std::max<int64_t>(64, round_up(maxr, 64));
+    const int opad = exchange_columns(maxr);
     cudaError_t e = pivoted_cholesky(b->D, b->nn, (int)b->n, kRankTolerance, maxr, b->Lc, b->nn, b->info, b->count,
                                      active, s);
     if (e != cudaSuccess) return e;
@@ -1045,7 +1045,7 @@ int hf_batch_exchange(hf_batch* b, const double* density, int64_t max_rank, doub
     if (!b || !density || !exchange || max_rank < 1) return HF_ERR_ARG;
     cudaSetDevice(b->device);
     const int maxr = (int)std::min<int64_t>(max_rank, b->n);
-    const int opad = (int)std::max<int64_t>(64, round_up(maxr, 64));
+    const int opad = exchange_columns(maxr);
     // one pivot beyond max_rank tells a density of higher rank from one of exactly max_rank
     const int probe = (int)std::min<int64_t>(maxr + 1, b->n);
     HB_CU(pivoted_cholesky(density, b->nn, (int)b->n, kRankTolerance, probe, b->Lc, b->nn, b->info, b->count,

@@ -212,12 +212,14 @@ const double* shared_boys_table(int device) {
     return tables[device];
 }
 
-// Page-locked error flags, one per live context: a kernel with bounded waits
-// writes its flag only when a wait runs out, so the host reads it after the
-// stream's synchronisation without a copy. One page for the process, kept until
-// it exits; a context that finds no free slot gets null and its builds use the
-// kernels that wait for nothing.
-constexpr int kFlagSlots = 1024;
+// Page-locked words that kernels write and the host reads after the stream's
+// synchronisation without a copy, a slot of 64 bytes per live context: word 0 is the
+// error flag of the one-pass Coulomb build (written only when a wait runs out), word
+// kFlagBf16 that of the last split-BF16 exchange, from word kFlagState on the state of
+// the last density factorisation. One block for the process, kept until it exits; a
+// context that finds no free slot gets null and uses copies and the kernels that wait
+// for nothing.
+constexpr int kFlagSlots = 1024, kFlagWords = 16, kFlagBf16 = 1, kFlagState = 4;
 std::mutex g_flag_mutex;
 int* g_flag_page = nullptr;
 std::vector<int> g_flag_free;
@@ -225,7 +227,8 @@ std::vector<int> g_flag_free;
 int* flag_slot() {
     std::lock_guard<std::mutex> lock(g_flag_mutex);
     if (!g_flag_page) {
-        if (cudaHostAlloc((void**)&g_flag_page, sizeof(int) * kFlagSlots, cudaHostAllocPortable) != cudaSuccess) {
+        if (cudaHostAlloc((void**)&g_flag_page, sizeof(int) * kFlagSlots * kFlagWords, cudaHostAllocPortable) !=
+            cudaSuccess) {
             cudaGetLastError();
             g_flag_page = nullptr;
             return nullptr;
@@ -233,7 +236,7 @@ int* flag_slot() {
         for (int i = kFlagSlots - 1; i >= 0; --i) g_flag_free.push_back(i);
     }
     if (g_flag_free.empty()) return nullptr;
-    int* p = g_flag_page + g_flag_free.back();
+    int* p = g_flag_page + g_flag_free.back() * kFlagWords;
     g_flag_free.pop_back();
     *p = 0;
     return p;
@@ -242,7 +245,38 @@ int* flag_slot() {
 void flag_release(int* p) {
     if (!p) return;
     std::lock_guard<std::mutex> lock(g_flag_mutex);
-    g_flag_free.push_back((int)(p - g_flag_page));
+    g_flag_free.push_back((int)((p - g_flag_page) / kFlagWords));
+}
+
+// The streams of destroyed contexts, kept for the next ones (at most kOwnStreams per
+// device): creating and destroying one took 160 us, a twelfth of a dimer's setup.
+constexpr size_t kOwnStreams = 64;
+std::mutex g_stream_mutex;
+std::vector<cudaStream_t> g_streams[64];
+
+cudaError_t take_stream(int device, cudaStream_t* out) {
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lock(g_stream_mutex);
+        if (!g_streams[device].empty()) {
+            *out = g_streams[device].back();
+            g_streams[device].pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+}
+
+// `stream` has been synchronised by its context.
+void give_stream(int device, cudaStream_t stream) {
+    if (!stream) return;
+    if (device >= 0 && device < 64) {
+        std::lock_guard<std::mutex> lock(g_stream_mutex);
+        if (g_streams[device].size() < kOwnStreams) {
+            g_streams[device].push_back(stream);
+            return;
+        }
+    }
+    cudaStreamDestroy(stream);
 }
 
 // Side streams for Branches: one set per device, kept until the process exits and
@@ -1127,9 +1161,11 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
     const size_t row_bytes = sizeof(double) * 4096 * (size_t)N * ctx->nt;  // the widest row
     size_t budget = std::max<size_t>(row_bytes, (size_t)4 << 30);
     budget = std::min<size_t>(budget, sizeof(double) * 4096 * (size_t)N * ctx->ntiles);
-    size_t freeb = 0, totalb = 0;
-    cudaMemGetInfo(&freeb, &totalb);
-    if (budget > freeb / 2) budget = std::max(row_bytes, freeb / 2);
+    if (budget > ((size_t)64 << 20)) {  // the driver's answer takes 100 us or more
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        if (budget > freeb / 2) budget = std::max(row_bytes, freeb / 2);
+    }
     std::vector<std::pair<int, int>> chunks;
     for (int row0 = 0; row0 < ctx->nt;) {
         int row1 = row0 + 1;
@@ -1330,11 +1366,17 @@ static int exchange_from_ct(hf_ctx* ctx, const double* Ct, int opad, const doubl
     if (precision != HF_PREC_FP64) return fail(ctx, HF_ERR_ARG, "unknown precision");
     const JkPlan p = plan_of(ctx);
     const int64_t npad = (int64_t)ctx->nt * 64;
-    // X chunk: npad x qchunk x opad doubles, within a budget
-    size_t freeb = 0, totalb = 0;
-    cudaMemGetInfo(&freeb, &totalb);
+    // X chunk: npad x qchunk x opad doubles, within a budget; the driver is asked for the free
+    // memory only when the scratch does not hold every row already
     const size_t per_q = sizeof(double) * npad * opad * (any_negative ? 2 : 1);
-    size_t budget = std::min<size_t>((size_t)4 << 30, freeb / 3);
+    const size_t fixed = sizeof(double) * ((size_t)round_up(npad * npad, 32) +
+                                           (size_t)round_up(syrk_partial_doubles(npad, 1), 32));
+    size_t budget = (size_t)4 << 30;
+    if (ctx->kscratch_bytes < fixed + std::min(budget, per_q * (size_t)p.naux)) {
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        budget = std::min<size_t>(budget, freeb / 3);
+    }
     int qchunk = (int)std::max<size_t>(1, std::min<size_t>(budget / per_q, (size_t)p.naux));
     qchunk = std::min(qchunk, 65535);
     const size_t kp_doubles = (size_t)round_up(npad * npad, 32);
@@ -1368,15 +1410,20 @@ static int exchange_bf16(hf_ctx* ctx, const TcPlan& t, const double* Ct_tc, doub
             return s;
         }
     }
-    size_t freeb = 0, totalb = 0;
-    cudaMemGetInfo(&freeb, &totalb);
     const size_t ct_bytes = 2 * 2 * (size_t)t.opad * t.npad;
     const size_t per_q = (sign ? 4 : 2) * 2 * (size_t)t.npad * t.opad;
     const size_t kp_doubles = (size_t)round_up(t.npad * t.npad, 32);
-    size_t budget = std::min<size_t>((size_t)2 << 30, freeb / 3);
-    size_t want = round_up((int64_t)ct_bytes, 256) + tc_partial_bytes(t.npad) +
-                  per_q * std::max<size_t>(1, std::min<size_t>(budget / per_q, (size_t)p.naux));
-    want = round_up((int64_t)want, 256) + sizeof(double) * kp_doubles;
+    auto wanted = [&](size_t budget) {
+        const size_t w = round_up((int64_t)ct_bytes, 256) + tc_partial_bytes(t.npad) +
+                         per_q * std::max<size_t>(1, std::min<size_t>(budget / per_q, (size_t)p.naux));
+        return (size_t)round_up((int64_t)w, 256) + sizeof(double) * kp_doubles;
+    };
+    size_t want = wanted((size_t)2 << 30);
+    if (ctx->tcwork_bytes < want) {
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        want = wanted(std::min<size_t>((size_t)2 << 30, freeb / 3));
+    }
     int st = ensure_scratch(ctx, &ctx->d_tcwork, &ctx->tcwork_bytes, want);
     if (st != HF_OK) return st;
     double* Kp = ctx->d_tcwork;
@@ -1403,7 +1450,7 @@ int hf_exchange_factored(hf_ctx* ctx, const double* C, int64_t ncols, const doub
     if (!ctx->built) return fail(ctx, HF_ERR_STATE, "build the fitted tensor first");
     cudaSetDevice(ctx->device);
     const int64_t n = ctx->n, npad = (int64_t)ctx->nt * 64;
-    const int64_t opad = std::max<int64_t>(64, round_up(ncols, 64));
+    const int64_t opad = exchange_columns(ncols);
     bool neg = false;
     std::vector<double> wh;
     const double* dC = C;
@@ -1613,18 +1660,17 @@ int hf_density_factor(hf_ctx* ctx, const double* D, double* F, int64_t max_rank,
         dD = sD;
     }
     time_begin(ctx);
-    HF_CU(cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), ctx->stream));
-    HF_CU(pivoted_cholesky_blocked(dD, (int)n, 1e-14, (int)cap, Lc, ctx->d_info, ctx->d_stage + oW, ctx->stream));
+    int indefinite = 0;
+    int64_t found = 0;
+    HF_CU(pivoted_cholesky_blocked(dD, (int)n, 1e-14, (int)cap, Lc, ctx->d_stage + oW, &found, &indefinite,
+                                   ctx->stream, ctx->h_flag ? ctx->h_flag + kFlagState : nullptr));
     ++ctx->stats.kernel_launches;
-    int res[2] = {0, 0};
-    HF_CU(cudaMemcpyAsync(res, ctx->d_info, sizeof(res), cudaMemcpyDeviceToHost, ctx->stream));
-    HF_CU(cudaStreamSynchronize(ctx->stream));
     ctx->stats.ms_factorize_density = time_end(ctx);
-    if (res[1])
+    if (indefinite)
         return fail(ctx, HF_ERR_NUMERIC, "the density is not positive semidefinite");
-    *rank = res[0];
+    *rank = found;
     if (!on_device) {
-        HF_CU(cudaMemcpyAsync(F, Lc, sizeof(double) * (size_t)res[0] * n, cudaMemcpyDeviceToHost, ctx->stream));
+        HF_CU(cudaMemcpyAsync(F, Lc, sizeof(double) * (size_t)found * n, cudaMemcpyDeviceToHost, ctx->stream));
         return check_async(ctx, "hf_density_factor");
     }
     return HF_OK;
@@ -1652,25 +1698,22 @@ int hf_exchange(hf_ctx* ctx, const double* D, double* K, int precision, int on_d
         dD = sD;
     }
     time_begin(ctx);
-    cudaMemsetAsync(ctx->d_info, 0, 2 * sizeof(int), ctx->stream);
-    HF_CU(pivoted_cholesky_blocked(dD, (int)n, 1e-14, (int)n, Lc, ctx->d_info, buf + oW, ctx->stream));
-    int res[2] = {0, 0};
-    cudaMemcpyAsync(res, ctx->d_info, sizeof(res), cudaMemcpyDeviceToHost, ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    int indefinite = 0;
+    int64_t rank = 0;
+    HF_CU(pivoted_cholesky_blocked(dD, (int)n, 1e-14, (int)n, Lc, buf + oW, &rank, &indefinite, ctx->stream,
+                                   ctx->h_flag ? ctx->h_flag + kFlagState : nullptr));
     ctx->stats.ms_factorize_density = time_end(ctx);
-    if (e != cudaSuccess) return fail(ctx, HF_ERR_CUDA, std::string("pivoted Cholesky: ") + cudaGetErrorString(e));
-    if (res[1])
+    if (indefinite)
         return fail(ctx, HF_ERR_NUMERIC, "the density is not positive semidefinite; pass a signed factor to "
                                          "hf_exchange_factored");
-    const int64_t rank = res[0];
     if (precision == HF_PREC_BF16X3) {
         const TcPlan t = tc_plan(n, fitted_rows(ctx), rank);
         int sc = ensure_scratch(ctx, &ctx->d_ctc, &ctx->ctc_bytes, sizeof(double) * ((size_t)t.opad * t.npad + t.opad));
         if (sc != HF_OK) return sc;
         double* Ct_tc = ctx->d_ctc;
         time_begin(ctx);
-        const cudaError_t fe = factor_pad(Lc, 0, n, ctx->d_info, Ct_tc, 0, t.npad, t.opad,
-                                          Ct_tc + (size_t)t.opad * t.npad, 1, nullptr, ctx->stream);
+        const cudaError_t fe = factor_pad(Lc, 0, n, nullptr, Ct_tc, 0, t.npad, t.opad,
+                                          Ct_tc + (size_t)t.opad * t.npad, 1, nullptr, ctx->stream, rank);
         double* dK = on_device ? K : sK;
         int s = fe == cudaSuccess ? exchange_bf16(ctx, t, Ct_tc, dK)
                                   : fail(ctx, HF_ERR_CUDA, std::string("factor_pad: ") + cudaGetErrorString(fe));
@@ -1680,11 +1723,11 @@ int hf_exchange(hf_ctx* ctx, const double* D, double* K, int precision, int on_d
         if (s == HF_OK) s = check_async(ctx, "hf_exchange");
         return s;
     }
-    const int64_t opad = std::max<int64_t>(64, round_up(rank, 64));
+    const int64_t opad = exchange_columns(rank);
     double* Ct = buf + oCt;
     double* sign = buf + osg;
     time_begin(ctx);
-    HF_CU(factor_pad(Lc, 0, n, ctx->d_info, Ct, 0, npad, opad, sign, 1, nullptr, ctx->stream));
+    HF_CU(factor_pad(Lc, 0, n, nullptr, Ct, 0, npad, opad, sign, 1, nullptr, ctx->stream, rank));
     double* dK = on_device ? K : sK;
     int s = exchange_from_ct(ctx, Ct, (int)opad, sign, false, dK, precision);
     if (s == HF_OK && !on_device) cudaMemcpyAsync(K, sK, sizeof(double) * nn, cudaMemcpyDeviceToHost, ctx->stream);

@@ -13,6 +13,7 @@
 //       GEMM over the q-chunk, only upper 64x64 output tiles computed.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 
 #include "dgemm.cuh"
@@ -171,10 +172,22 @@ __global__ void k_symmetrize_upper(const double* __restrict__ Kp, int64_t ldk, i
 // were 4 % slower). The A operand comes from the packed tiles: tile (Ip, J) when
 // Ip <= J, else tile (J, Ip) read in its own orientation and transposed by the
 // fragment loads.
-constexpr int XBM = 64, XBN = 64, XBK = 32, XLD = XBK + 4, XST = 2, XTHREADS = 128;
+// The column tile is 32, 48, 64 or 80 wide, whichever pads the factor least: 160
+// orbitals are two tiles of 80, not three of 64, and the 10 of a water dimer one of
+// 32. 80-wide tiles keep three CTAs per SM with 3 stages of 16-wide slices.
+constexpr int XBM = 64;
 constexpr int XLDT = 64 + 4;  // pitch of a k-major half: conflict-free fragment loads
-static_assert(XBK * XLDT <= 64 * XLD, "a k-major half fits in the p-major half's space");
-static_assert(XBM % 64 == 0 && 64 % XBK == 0, "a k slice stays inside one packed tile");
+template <int XBN>
+struct HalfShape {
+    static constexpr int BK = XBN == 80 ? 16 : 32, ST = XBN == 80 ? 3 : 2, LD = BK + 4;
+    static constexpr int NW = XBN == 32 ? 1 : 2;   // warps along the columns
+    static constexpr int WN = XBN / NW, J = WN / 8;  // a warp: 32 x WN outputs
+    static constexpr int THREADS = 64 * NW;
+    static constexpr int SMEM = ST * (XBM + XBN) * LD * (int)sizeof(double);
+    static_assert(BK * XLDT <= 64 * LD, "a k-major half fits in the p-major half's space");
+    static_assert(64 % BK == 0, "a k slice stays inside one packed tile");
+    static_assert(WN % 8 == 0 && (XBN * BK / 2) % THREADS == 0, "whole mma tiles and copies");
+};
 
 __device__ __forceinline__ uint32_t xsmem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -192,12 +205,16 @@ __device__ __forceinline__ void xmma(double (&c)[4], const double (&a)[4], const
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-__global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* const* __restrict__ Btab,
+template <int XBN>
+__global__ void __launch_bounds__(HalfShape<XBN>::THREADS, 3) k_exchange_half(const double* const* __restrict__ Btab,
                                                              const double* __restrict__ B, int64_t ldb, int q0, int nt,
                                                              const double* __restrict__ Ct, int64_t ldc_t,
-                                                             int64_t strideCt, int npad, double* __restrict__ X,
+                                                             int64_t strideCt, int n, int npad,
+                                                             double* __restrict__ X,
                                                              int64_t ldx, int64_t strideX, int opad,
                                                              const int* __restrict__ active, int transposed) {
+    using SH = HalfShape<XBN>;
+    constexpr int XBK = SH::BK, XST = SH::ST, XLD = SH::LD, XTHREADS = SH::THREADS, J = SH::J;
     const int row_tiles = (npad + XBM - 1) / XBM;
     const int cl = blockIdx.y / row_tiles;
     if (active && active[cl] == 0) return;
@@ -212,21 +229,23 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
     double* Bs = xs + XST * XBM * XLD;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gq = lane >> 2, tq = lane & 3;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int nk = npad / XBK;
+    const int wm = warp / SH::NW * 32, wn = warp % SH::NW * SH::WN;
+    const int nk = (n + XBK - 1) / XBK;  // B_q is zero past n
+    // a warp whose rows are all past n, or whose columns are all past the factor's, only loads
+    const bool live = m0 + wm < n && n0 + wn < opad;
 
     // Each stage holds the A rows as two 64-row halves. A half whose tile lies on
     // or above the diagonal (Ip <= J) is stored p-major ([p][k], pitch XLD) from
     // tile (Ip, J); a half below it reads tile (J, Ip), where k is the slow index,
     // and is stored k-major ([k][p], pitch XLDT) so that both the global reads and
     // the shared writes are contiguous; the fragment loads read it transposed.
-    auto tile_at = [&](int I, int Jt) -> const double* {
-        return Bq + ((int64_t)I * nt - (int64_t)I * (I - 1) / 2 + (Jt - I)) * 4096;
+    auto tile_at = [&](int I, int Jc) -> const double* {
+        return Bq + ((int64_t)I * nt - (int64_t)I * (I - 1) / 2 + (Jc - I)) * 4096;
     };
     auto load = [&](int stage, int k0) {
         double* as = As + stage * XBM * XLD;
         double* bs = Bs + stage * XBN * XLD;
-        const int J = k0 >> 6, kin = k0 & 63;
+        const int Jt = k0 >> 6, kin = k0 & 63;
         constexpr int PIECES = 64 * XBK / 2;  // 16-byte pieces of a 64 x XBK half
 #pragma unroll
         for (int h = 0; h < XBM / 64; ++h) {
@@ -234,8 +253,8 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
             const int Ip = p0 >> 6;
             double* ah = as + h * 64 * XLD;
             const bool valid = p0 < npad;
-            const bool below = Ip > J;
-            const double* tile = valid ? (below ? tile_at(J, Ip) : tile_at(Ip, J)) : Bq;
+            const bool below = Ip > Jt;
+            const double* tile = valid ? (below ? tile_at(Jt, Ip) : tile_at(Ip, Jt)) : Bq;
 #pragma unroll
             for (int c = 0; c < PIECES / XTHREADS; ++c) {
                 const int e = tid + c * XTHREADS;
@@ -252,15 +271,15 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
         for (int c = 0; c < XBN * XBK / 2 / XTHREADS; ++c) {
             const int e = tid + c * XTHREADS;  // the 16-byte pieces of the XBN x XBK tile of Ct
             const int r = e / (XBK / 2), kp = (e % (XBK / 2)) * 2;
-            xcp16(bs + r * XLD + kp, Ct + (int64_t)(n0 + r) * ldc_t + k0 + kp, Ct, true);
+            xcp16(bs + r * XLD + kp, Ct + (int64_t)(n0 + r) * ldc_t + k0 + kp, Ct, n0 + r < opad);
         }
     };
 
-    double acc[2][4][4];
+    double acc[2][J][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < J; ++j)
 #pragma unroll
             for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
 #pragma unroll
@@ -280,9 +299,10 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
         const int hh = wm >> 6, lr = wm & 63;
         const bool below = ((m0 >> 6) + hh) > ((it * XBK) >> 6);
         const double* ah = as + hh * 64 * XLD;
+        if (!live) continue;
 #pragma unroll
         for (int kk = 0; kk < XBK; kk += 8) {
-            double af[2][4], bf[4][2];
+            double af[2][4], bf[J][2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int row = lr + i * 16 + gq;
@@ -301,7 +321,7 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < J; ++j) {
                 const double* c0 = bs + (wn + j * 8 + gq) * XLD + kk + tq;
                 bf[j][0] = c0[0];
                 bf[j][1] = c0[4];
@@ -309,7 +329,7 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) xmma(acc[i][j], af[i], bf[j]);
+                for (int j = 0; j < J; ++j) xmma(acc[i][j], af[i], bf[j]);
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::);
@@ -319,12 +339,12 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < J; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int m = m0 + wm + i * 16 + gq + h * 8;
                     const int nn = n0 + wn + j * 8 + 2 * tq;
-                    if (m < npad) {
+                    if (m < npad && nn < opad) {
                         xt[(int64_t)nn * npad + m] = acc[i][j][2 * h];
                         xt[(int64_t)(nn + 1) * npad + m] = acc[i][j][2 * h + 1];
                     }
@@ -335,12 +355,12 @@ __global__ void __launch_bounds__(XTHREADS, 3) k_exchange_half(const double* con
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < J; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int m = m0 + wm + i * 16 + gq + h * 8;
                 const int nn = n0 + wn + j * 8 + 2 * tq;
-                if (m < npad)
+                if (m < npad && nn < opad)
                     *reinterpret_cast<double2*>(xo + (int64_t)m * ldx + nn) = make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
             }
 }
@@ -453,145 +473,151 @@ __global__ void __launch_bounds__(1024) k_pivoted_cholesky(const double* __restr
 }
 
 // Blocked pivoted Cholesky of one matrix: the pivots and the factor of
-// k_pivoted_cholesky, with the rows that pivots already taken subtract kept in
-// a working copy W = D - sum L L^T that a DMMA product updates once per panel
-// of kPivotPanel pivots. Within a panel each pivot's column needs W's row and
-// at most kPivotPanel - 1 corrections instead of one per earlier pivot, so the
-// sequential part no longer rereads the whole factor from L2 at every pivot.
-constexpr int kPivotPanel = 32;
+// k_pivoted_cholesky up to rounding, with the rows that pivots already taken
+// subtract kept in a working copy W = D - sum L L^T that a DMMA product updates
+// once per panel.
+//
+// A panel is one CTA's chain of pivots, so a pivot's latency is what counts. The
+// panel's rows of L sit in shared memory (as many pivots per panel as fit: all of
+// them up to n = 160, 94 at n = 288, 16 at n = 1536), the pivot is found with one
+// barrier (64-bit keys of value and index, reduced by two 32-bit warp reductions
+// each), the pivot's row of W is on its way while the corrections are summed, and
+// no division is in the chain. Per pivot about 0.6 us, where the rows of L in
+// global memory and two shuffled reductions took 4 (n = 48) to 20 us (n = 1536).
 struct PivotState {
     double dmax0;  // the largest initial diagonal entry
     int k;         // pivots taken
     int stop;      // 1 once the remaining diagonal falls below tol dmax0 or k reaches maxr
+    int bad;       // 1 when a remaining diagonal entry is clearly negative (set with stop)
     int active;    // the trailing update of this panel has work (DMMA batch flag)
-    int pad;
 };
 
-__device__ __forceinline__ void block_argmax(double best, int bi, double* rv, int* ri, double& out_best,
-                                             int& out_i) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi >= 0 && (bi < 0 || oi < bi))) {
-            best = ob;
-            bi = oi;
-        }
-    }
-    if ((threadIdx.x & 31) == 0) {
-        rv[threadIdx.x >> 5] = best;
-        ri[threadIdx.x >> 5] = bi;
-    }
-    __syncthreads();
-    double b = -1.0;
-    int p = -1;
-    for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w)
-        if (rv[w] > b || (rv[w] == b && ri[w] >= 0 && (p < 0 || ri[w] < p))) {
-            b = rv[w];
-            p = ri[w];
-        }
-    out_best = b;
-    out_i = p;
+// The largest 64-bit key of a warp, in every lane.
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long key) {
+    const unsigned hi = (unsigned)(key >> 32);
+    const unsigned top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned low = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)key : 0u);
+    return ((unsigned long long)top << 32) | low;
 }
 
-__global__ void __launch_bounds__(1024) k_pc_init(const double* __restrict__ D, int n, double* __restrict__ d,
-                                                  unsigned char* __restrict__ used, PivotState* st) {
-    __shared__ double rv[32];
-    __shared__ int ri[32];
-    double m = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        d[i] = D[(int64_t)i * n + i];
-        used[i] = 0;
-        m = fmax(m, fabs(d[i]));
-    }
-    double b;
-    int unused_i;
-    block_argmax(m, (int)threadIdx.x, rv, ri, b, unused_i);
-    if (threadIdx.x == 0) {
-        st->dmax0 = b;
-        st->k = 0;
-        st->stop = n > 0 ? 0 : 1;
-        st->active = 0;
-    }
-}
+constexpr int kPivotThreads = 1024;
+constexpr int kPivotRows = 22;  // rows per thread (n <= 22528)
 
-__global__ void __launch_bounds__(512) k_pc_panel(const double* __restrict__ W, int n, double tol, int maxr,
-                                                   double* __restrict__ Lc, double* __restrict__ Lp,
-                                                   double* __restrict__ d, unsigned char* __restrict__ used,
-                                                   PivotState* st) {
-    __shared__ double rv[32];
-    __shared__ int ri[32];
-    __shared__ double s_piv;
-    __shared__ int s_p, s_stop;
-    const int tid = threadIdx.x;
-    const int k0 = st->k;
-    const double dmax0 = st->dmax0;
-    if (st->stop) {
-        if (tid == 0) st->active = 0;
+// One panel of up to `width` pivots of W (D itself for the first). Shared: d[n],
+// Lp[n][pitch] when it fits (else Lp is the global copy).
+__global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __restrict__ W, int n, double tol, int maxr,
+                                                            double* __restrict__ Lc, double* __restrict__ Lg,
+                                                            int width, int pitch, int in_smem,
+                                                            double* __restrict__ dg, unsigned char* __restrict__ used,
+                                                            int first, PivotState* st, PivotState* host) {
+    extern __shared__ double psm[];
+    __shared__ unsigned long long keys[2][32];
+    __shared__ int s_bad;
+    double* d = psm;
+    double* Lp = in_smem ? psm + n : Lg;
+    const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, warps = T >> 5;
+    if (!first && st->stop) {
+        if (tid == 0) {
+            st->active = 0;
+            if (host) *host = *st;
+        }
         return;
     }
-    const int b = min(kPivotPanel, maxr - k0);
-    int done = 0;
-    for (int j = 0; j < b; ++j) {
-        double best = -1.0;
-        int bi = -1;
-        for (int i = tid; i < n; i += blockDim.x)
-            if (!used[i] && d[i] > best) {
-                best = d[i];
-                bi = i;
-            }
-        double bb;
-        int p;
-        block_argmax(best, bi, rv, ri, bb, p);
-        if (tid == 0) {
-            s_stop = (p < 0 || !(bb > tol * dmax0)) ? 1 : 0;
-            s_p = p;
-            s_piv = s_stop ? 0.0 : sqrt(bb);
-        }
+    unsigned mine = 0;  // bit m: row tid + m T has been a pivot
+    double top = 0.0;
+    for (int i = tid, m = 0; i < n; i += T, ++m) {
+        const double v = first ? W[(int64_t)i * n + i] : dg[i];
+        d[i] = v;
+        if (first) top = fmax(top, fabs(v));
+        else if (used[i]) mine |= 1u << m;
+    }
+    if (tid == 0) s_bad = 0;
+    double dmax0;
+    if (first) {
+        const unsigned long long k = warp_max_key((unsigned long long)__double_as_longlong(top));
+        if (lane == 0) keys[1][warp] = k;
         __syncthreads();
-        if (s_stop) break;
-        const int pv = s_p;
-        const double piv = s_piv;
-        // each thread owns rows i = tid + m blockDim.x: it alone writes their column
-        // entries, diagonal and used flag, and alone reads d and used for them in
-        // the next pivot's search, so the two barriers of the search suffice
-        for (int i = tid; i < n; i += blockDim.x) {
+        dmax0 = __longlong_as_double((long long)warp_max_key(lane < warps ? keys[1][lane] : 0ull));
+        __syncthreads();
+    } else {
+        dmax0 = st->dmax0;
+        __syncthreads();
+    }
+    const int k0 = first ? 0 : st->k;
+    const int b = min(width, maxr - k0);
+    int j = 0;
+    for (; j < b; ++j) {
+        // the largest remaining diagonal entry, the lowest index among those equal to 2^-36 of it
+        unsigned long long key = 0;
+        for (int i = tid, m = 0; i < n; i += T, ++m)
+            if (!(mine >> m & 1) && d[i] > 0.0) {
+                const unsigned long long k =
+                    ((unsigned long long)__double_as_longlong(d[i]) & ~0xffffull) | (unsigned long long)(0xffff - i);
+                key = k > key ? k : key;
+            }
+        key = warp_max_key(key);
+        if (lane == 0) keys[j & 1][warp] = key;
+        __syncthreads();
+        key = warp_max_key(lane < warps ? keys[j & 1][lane] : 0ull);
+        const int p = key ? 0xffff - (int)(key & 0xffff) : 0;
+        const double best = key ? d[p] : 0.0;
+        if (!(best > tol * dmax0)) break;
+        const double piv = sqrt(best), inv = 1.0 / piv;
+        const double* __restrict__ w = W + (int64_t)p * n;
+        const double* lp = Lp + (int64_t)p * pitch;
+        // each thread owns rows i = tid + m T: it alone writes their entries of L, their diagonal and their
+        // used bit, so the search's barrier suffices
+        for (int i = tid, m = 0; i < n; i += T, ++m) {
             double l = 0.0;
-            if (i == pv) {
+            if (i == p) {
                 l = piv;
-                used[i] = 1;
-            } else if (!used[i]) {
-                double sum = W[(int64_t)pv * n + i];
-                for (int jj = 0; jj < j; ++jj) sum -= Lp[i * kPivotPanel + jj] * Lp[pv * kPivotPanel + jj];
-                l = sum / piv;
+                mine |= 1u << m;
+            } else if (!(mine >> m & 1)) {
+                const double wi = w[i];
+                const double* li = Lp + (int64_t)i * pitch;
+                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+                int q = 0;
+                for (; q + 3 < j; q += 4) {
+                    s0 += li[q] * lp[q];
+                    s1 += li[q + 1] * lp[q + 1];
+                    s2 += li[q + 2] * lp[q + 2];
+                    s3 += li[q + 3] * lp[q + 3];
+                }
+                for (; q < j; ++q) s0 += li[q] * lp[q];
+                const double s = wi - ((s0 + s1) + (s2 + s3));
+                l = s * inv;
+                l = fma(inv, fma(-l, piv, s), l);  // s / piv
                 d[i] -= l * l;
             }
             Lc[(int64_t)(k0 + j) * n + i] = l;
-            Lp[i * kPivotPanel + j] = l;
+            Lp[(int64_t)i * pitch + j] = l;
         }
-        ++done;
     }
     __syncthreads();
-    // columns of the panel past its last pivot add nothing to the trailing update
-    for (int e = tid; e < n * kPivotPanel; e += blockDim.x)
-        if (e % kPivotPanel >= done) Lp[e] = 0.0;
-    if (tid == 0) {
-        st->k = k0 + done;
-        st->stop = (done < b || k0 + done >= maxr) ? 1 : 0;
-        st->active = done > 0 ? 1 : 0;
-    }
-}
-
-__global__ void __launch_bounds__(1024) k_pc_finish(int n, double tol, const double* __restrict__ d,
-                                                    const unsigned char* __restrict__ used,
-                                                    const PivotState* st, int* __restrict__ out) {
-    // indefinite if a remaining diagonal entry is clearly negative
+    const bool stop = j < b || k0 + j >= maxr;
     int bad = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (!used[i] && d[i] < -1e3 * tol * st->dmax0) bad = 1;
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) {
-        out[0] = st->k;
-        out[1] = bad;
+    for (int i = tid, m = 0; i < n; i += T, ++m) {
+        const bool u = mine >> m & 1;
+        dg[i] = d[i];
+        used[i] = u;
+        // indefinite if a remaining diagonal entry is clearly negative
+        if (stop && !u && d[i] < -1e3 * tol * dmax0) bad = 1;
+    }
+    if (bad) s_bad = 1;
+    // the panel for the trailing update; columns past its last pivot add nothing to it
+    if (!stop)
+        for (int e = tid; e < n * width; e += T) {
+            const int i = e / width, c = e - i * width;
+            Lg[e] = c < j ? Lp[(int64_t)i * pitch + c] : 0.0;
+        }
+    __syncthreads();
+    if (tid == 0) {
+        st->dmax0 = dmax0;
+        st->k = k0 + j;
+        st->stop = stop ? 1 : 0;
+        st->bad = s_bad;
+        st->active = stop ? 0 : 1;
+        if (host) *host = *st;
     }
 }
 
@@ -599,12 +625,12 @@ __global__ void __launch_bounds__(1024) k_pc_finish(int n, double tol, const dou
 // sign[i] = 1 when sign is given (single cluster).
 __global__ void k_factor_pad(const double* __restrict__ Lc, int64_t strideL, int64_t n, const int* __restrict__ info,
                              double* __restrict__ Ct, int64_t strideCt, int64_t npad, int64_t opad,
-                             double* __restrict__ sign, const int* __restrict__ active) {
+                             double* __restrict__ sign, const int* __restrict__ active, int64_t known_rank) {
     const int cl = blockIdx.y;
     if (active && active[cl] == 0) return;
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= opad * npad) return;
-    const int64_t rank = info[2 * cl];
+    const int64_t rank = info ? info[2 * cl] : known_rank;
     const int64_t i = e / npad, mu = e % npad;
     Ct[cl * strideCt + e] = (i < rank && mu < n) ? Lc[cl * strideL + i * n + mu] : 0.0;
     if (sign && mu == 0) sign[i] = 1.0;
@@ -621,6 +647,24 @@ __global__ void k_sum_splits(const double* __restrict__ P, int splits, int64_t n
     double s = 0.0;
     for (int k = 0; k < splits; ++k) s += src[(int64_t)k * nn];
     Kp[(int64_t)c * nn + e] += s;
+}
+
+// K of one chunk of rows straight from its partial products: K[mu][nu] = K[nu][mu] =
+// sum_s P[c][s][min][max] in split order, eight loads at a time.
+__global__ void k_sum_splits_symmetric(const double* __restrict__ P, int splits, int64_t ldk, int64_t n,
+                                       double* __restrict__ K, int64_t strideK, const int* __restrict__ active) {
+    const int c = blockIdx.y;
+    if (active && active[c] == 0) return;
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n * n) return;
+    const int64_t mu = e / n, nu = e % n;
+    if (mu > nu) return;
+    const double* src = P + (int64_t)c * splits * ldk * ldk + mu * ldk + nu;
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) s += src[(int64_t)k * ldk * ldk];
+    K[c * strideK + e] = s;
+    K[c * strideK + nu * n + mu] = s;
 }
 
 constexpr int kMaxDevices = 64;
@@ -695,6 +739,28 @@ int64_t syrk_partial_doubles(int64_t npad, int count) {
     return s > 1 ? (int64_t)s * std::max(1, count) * npad * npad : 0;
 }
 
+namespace {
+template <int XBN>
+cudaError_t launch_half_as(const JkPlan& p, int q0, int qc, const double* Ct, int64_t strideCt, int64_t npad, double* X,
+                           int64_t ldx, int64_t strideX, int opad, int transposed, cudaStream_t stream) {
+    dim3 grid((opad + XBN - 1) / XBN, (unsigned)(((npad + XBM - 1) / XBM) * p.count), qc);
+    k_exchange_half<XBN><<<grid, HalfShape<XBN>::THREADS, HalfShape<XBN>::SMEM, stream>>>(
+        p.Btab, p.B, p.ldb, q0, p.nt, Ct, npad, strideCt, (int)p.n, (int)npad, X, ldx, strideX, opad, p.active, transposed);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_half(const JkPlan& p, int q0, int qc, const double* Ct, int64_t strideCt, int64_t npad, double* X,
+                        int64_t ldx, int64_t strideX, int opad, int transposed, cudaStream_t stream) {
+    // the least padded width; on a tie the wider of 64 and 32, then 80 and 48
+    int best = 64;
+    for (int w : {32, 80, 48})
+        if ((opad + w - 1) / w * w < (opad + best - 1) / best * best) best = w;
+    auto run = best == 32 ? launch_half_as<32> : best == 48 ? launch_half_as<48> : best == 80 ? launch_half_as<80>
+                                                                                             : launch_half_as<64>;
+    return run(p, q0, qc, Ct, strideCt, npad, X, ldx, strideX, opad, transposed, stream);
+}
+}  // namespace
+
 cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int64_t strideCt, int opad, const double* sign,
                                 double* K, int64_t strideK, double* Kp, double* X, double* Xs, double* partial,
                                 int qchunk, cudaStream_t stream) {
@@ -702,16 +768,15 @@ cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int64_t strid
     if (sign != nullptr && p.count != 1) return cudaErrorInvalidValue;
     cudaError_t e = jk_configure();
     if (e != cudaSuccess) return e;
-    cudaMemsetAsync(Kp, 0, sizeof(double) * npad * npad * p.count, stream);
-    const int smem = XST * (XBM + XBN) * XLD * (int)sizeof(double);
-    const int row_tiles = (int)((npad + XBM - 1) / XBM);
+    const int splits_wanted = partial ? syrk_splits(npad, p.count) : 1;
+    const bool direct = qchunk >= p.naux && splits_wanted > 1;  // one chunk: no running sum in Kp
+    if (!direct) cudaMemsetAsync(Kp, 0, sizeof(double) * npad * npad * p.count, stream);
     const int64_t strideX = npad * (int64_t)qchunk * opad;
     for (int q0 = 0; q0 < p.naux; q0 += qchunk) {
         const int qc = (p.naux - q0 < qchunk) ? p.naux - q0 : qchunk;
         const int64_t ldx = (int64_t)qc * opad;
-        dim3 grid(opad / 64, (unsigned)(row_tiles * p.count), qc);
-        k_exchange_half<<<grid, XTHREADS, smem, stream>>>(p.Btab, p.B, p.ldb, q0, p.nt, Ct, npad, strideCt, (int)npad, X,
-                                                          ldx, strideX, opad, p.active, 0);
+        e = launch_half(p, q0, qc, Ct, strideCt, npad, X, ldx, strideX, opad, 0, stream);
+        if (e != cudaSuccess) return e;
         const double* Xb = X;
         if (sign != nullptr) {
             const int64_t tot = npad * ldx;
@@ -719,7 +784,7 @@ cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int64_t strid
             Xb = Xs;
         }
         GemmArgs g{};
-        g.M = g.N = (int)npad;
+        g.M = g.N = (int)p.n;
         g.K = (int)ldx;
         g.A = X;
         g.lda = ldx;
@@ -735,7 +800,7 @@ cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int64_t strid
         g.strideA = g.strideB = strideX;
         g.strideC = npad * npad;
         g.active = p.active;
-        const int splits = partial ? syrk_splits(npad, p.count) : 1;
+        const int splits = splits_wanted;
         if (splits > 1) {
             // partial products per split, then a fixed-order sum into Kp
             g.C = partial;
@@ -743,6 +808,11 @@ cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int64_t strid
             g.splits = splits;
             e = dgemm_nt(g, p.count, stream);
             if (e != cudaSuccess) return e;
+            if (direct) {
+                k_sum_splits_symmetric<<<dim3((unsigned)((p.n * p.n + 255) / 256), (unsigned)p.count), 256, 0, stream>>>(
+                    partial, splits, npad, p.n, K, strideK, p.active);
+                return cudaGetLastError();
+            }
             const int64_t nn2 = npad * npad;
             k_sum_splits<<<dim3((unsigned)((nn2 + 255) / 256), (unsigned)p.count), 256, 0, stream>>>(
                 partial, splits, nn2, Kp, p.active);
@@ -767,52 +837,90 @@ cudaError_t pivoted_cholesky(const double* D, int64_t strideD, int n, double tol
     return cudaGetLastError();
 }
 
+namespace {
+// Pivots per panel and the pitch of its rows in shared memory (odd: rows of
+// consecutive threads in different banks); in_smem 0: rows in global memory.
+void pivot_panel(int n, int& width, int& pitch, int& in_smem) {
+    const int room = (int)((kPivotSmem - sizeof(double) * (size_t)n) / (sizeof(double) * (size_t)n));
+    in_smem = room >= 9;
+    pitch = in_smem ? std::min((room & 1) ? room : room - 1, n | 1) : 32;
+    width = in_smem ? std::max(1, std::min(pitch - 1, 256)) : 32;
+    if (n == 1) width = 1;
+}
+}  // namespace
+
+static_assert(sizeof(PivotState) <= kPivotMapped, "the mapped state's room");
+
 size_t pivoted_cholesky_work_doubles(int n) {
-    return (size_t)n * n + (size_t)n * kPivotPanel + n + (n + 7) / 8 + 4;
+    int width, pitch, in_smem;
+    pivot_panel(n, width, pitch, in_smem);
+    return (size_t)n * n + (size_t)n * std::max(width, pitch) + n + (n + 7) / 8 + 4;
 }
 
-cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, int* info,
-                                     double* work, cudaStream_t stream) {
-    if (n < 1 || maxr < 1) return cudaErrorInvalidValue;
+cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, double* work,
+                                     int64_t* rank, int* indefinite, cudaStream_t stream, void* mapped) {
+    if (n < 1 || maxr < 1 || n > kPivotThreads * kPivotRows) return cudaErrorInvalidValue;
     cudaError_t e = jk_configure();
     if (e != cudaSuccess) return e;
+    int width, pitch, in_smem;
+    pivot_panel(n, width, pitch, in_smem);
     double* W = work;
-    double* Lp = W + (size_t)n * n;
-    double* d = Lp + (size_t)n * kPivotPanel;
+    double* Lg = W + (size_t)n * n;
+    double* d = Lg + (size_t)n * std::max(width, pitch);
     unsigned char* used = reinterpret_cast<unsigned char*>(d + n);
     PivotState* st = reinterpret_cast<PivotState*>(d + n + (n + 7) / 8);
-    e = cudaMemcpyAsync(W, D, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, stream);
-    if (e != cudaSuccess) return e;
-    k_pc_init<<<1, 1024, 0, stream>>>(D, n, d, used, st);
-    const int panels = (maxr + kPivotPanel - 1) / kPivotPanel;
-    for (int pnl = 0; pnl < panels; ++pnl) {
-        k_pc_panel<<<1, 512, 0, stream>>>(W, n, tol, maxr, Lc, Lp, d, used, st);
-        if (pnl + 1 == panels) break;  // no pivot follows the last panel
-        // W -= Lp Lp^T (skipped, CTA by CTA, once the factorisation has stopped)
-        GemmArgs g{};
-        g.M = g.N = n;
-        g.K = kPivotPanel;
-        g.A = g.B = Lp;
-        g.lda = g.ldb = kPivotPanel;
-        g.C = W;
-        g.ldc = n;
-        g.alpha = -1.0;
-        g.beta = 1.0;
-        g.kmode = 0;
-        g.epi = 0;
-        g.tile = 5;
-        g.active = &st->active;
-        e = dgemm_nt(g, 1, stream);
+    const size_t smem = sizeof(double) * ((size_t)n + (in_smem ? (size_t)n * pitch : 0));
+    const int threads = std::min(kPivotThreads, std::max(128, (n + 31) / 32 * 32));
+    const int panels = (maxr + width - 1) / width;
+    // A density's rank is its occupied orbitals, about a fifth of n: panels for 0.3 n are queued
+    // before the first look at the state, the rest only when it has not stopped by then.
+    int queued = 0, until = std::max(1, std::min(panels, (int)(0.3 * n / width) + 1));
+    PivotState host{};
+    for (;;) {
+        for (; queued < until; ++queued) {
+            if (queued > 0) {
+                if (queued == 1) {
+                    e = cudaMemcpyAsync(W, D, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, stream);
+                    if (e != cudaSuccess) return e;
+                }
+                // W -= Lp Lp^T (skipped, CTA by CTA, once the factorisation has stopped)
+                GemmArgs g{};
+                g.M = g.N = n;
+                g.K = width;
+                g.A = g.B = Lg;
+                g.lda = g.ldb = width;
+                g.C = W;
+                g.ldc = n;
+                g.alpha = -1.0;
+                g.beta = 1.0;
+                g.kmode = 0;
+                g.epi = 0;
+                g.tile = 5;
+                g.active = &st->active;
+                e = dgemm_nt(g, 1, stream);
+                if (e != cudaSuccess) return e;
+            }
+            k_pc_panel<<<1, threads, smem, stream>>>(queued == 0 ? D : W, n, tol, maxr, Lc, Lg, width, pitch, in_smem, d,
+                                                     used, queued == 0 ? 1 : 0, st,
+                                                     queued + 1 == until ? static_cast<PivotState*>(mapped) : nullptr);
+        }
+        e = mapped ? cudaSuccess : cudaMemcpyAsync(&host, st, sizeof(host), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return e;
+        if (mapped) std::memcpy(&host, mapped, sizeof(host));
+        if (host.stop || queued >= panels) break;
+        until = panels;
     }
-    k_pc_finish<<<1, 1024, 0, stream>>>(n, tol, d, used, st, info);
+    *rank = host.k;
+    *indefinite = host.bad;
     return cudaGetLastError();
 }
 
 cudaError_t factor_pad(const double* Lc, int64_t strideL, int64_t n, const int* info, double* Ct, int64_t strideCt,
-                       int64_t npad, int64_t opad, double* sign, int count, const int* active, cudaStream_t stream) {
+                       int64_t npad, int64_t opad, double* sign, int count, const int* active, cudaStream_t stream,
+                       int64_t rank) {
     k_factor_pad<<<dim3((unsigned)((opad * npad + 255) / 256), (unsigned)count), 256, 0, stream>>>(
-        Lc, strideL, n, info, Ct, strideCt, npad, opad, sign, active);
+        Lc, strideL, n, info, Ct, strideCt, npad, opad, sign, active, rank);
     return cudaGetLastError();
 }
 
@@ -821,12 +929,9 @@ cudaError_t half_transform_t(const JkPlan& p, const double* Ct, int opad, int q0
     if (p.count != 1) return cudaErrorInvalidValue;
     cudaError_t e = jk_configure();
     if (e != cudaSuccess) return e;
-    const int64_t npad = (int64_t)p.nt * 64;
-    const int smem = XST * (XBM + XBN) * XLD * (int)sizeof(double);
-    dim3 grid(opad / 64, (unsigned)((npad + XBM - 1) / XBM), qc);
-    k_exchange_half<<<grid, XTHREADS, smem, stream>>>(p.Btab, p.B, p.ldb, q0, p.nt, Ct, npad, 0, (int)npad, Xt, 0, 0,
-                                                      opad, nullptr, 1);
-    return cudaGetLastError();
+    JkPlan all = p;
+    all.active = nullptr;
+    return launch_half(all, q0, qc, Ct, 0, (int64_t)p.nt * 64, Xt, 0, 0, opad, 1, stream);
 }
 
 cudaError_t jk_configure() {
@@ -836,10 +941,17 @@ cudaError_t jk_configure() {
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(g_jk_mutex);
     if (g_jk_configured[dev]) return cudaSuccess;
-    const int smem = XST * (XBM + XBN) * XLD * (int)sizeof(double);
-    e = cudaFuncSetAttribute(k_exchange_half, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(k_exchange_half<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, HalfShape<32>::SMEM);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_exchange_half<48>, cudaFuncAttributeMaxDynamicSharedMemorySize, HalfShape<48>::SMEM);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_exchange_half<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, HalfShape<64>::SMEM);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_exchange_half<80>, cudaFuncAttributeMaxDynamicSharedMemorySize, HalfShape<80>::SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_pivoted_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmem);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_pc_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmem);
     if (e != cudaSuccess) return e;
     g_jk_configured[dev] = true;
     return dgemm_configure();

@@ -34,7 +34,7 @@ int64_t coulomb_work_doubles(const JkPlan& p);  // per cluster
 cudaError_t fitted_charges(const JkPlan& p, const double* D, double* d, double* work, cudaStream_t stream);
 
 // K = sum_q (B_q C) diag(sign) (B_q C)^T. Ct: [opad][npad] (C^T, zero padded,
-// opad a multiple of 64). sign: [opad] or null for all +1 (single cluster only).
+// opad a multiple of 16). sign: [opad] or null for all +1 (single cluster only).
 // Kp: npad x npad scratch; X, Xs: npad x (qchunk * opad) scratch (Xs only when
 // sign != null); partial: syrk_partial_doubles(npad, count) doubles (may be null
 // when that is 0). Per cluster c: Ct + c strideCt, K + c strideK, Kp + c npad^2,
@@ -47,6 +47,10 @@ inline cudaError_t exchange_build_fp64(const JkPlan& p, const double* Ct, int op
                                        cudaStream_t stream) {
     return exchange_build_fp64(p, Ct, 0, opad, sign, K, 0, Kp, X, Xs, partial, qchunk, stream);
 }
+
+// The factor's columns padded for exchange_build_fp64: to 16 (the k slices of X X^T;
+// 64 columns for the 10 orbitals of a small molecule were most of its K build).
+inline int exchange_columns(int64_t ncols) { return (int)((ncols < 1 ? 1 : ncols) + 15) / 16 * 16; }
 
 // Split-K factor of the K = X X^T product for `count` clusters of padded size
 // npad (enough CTAs for about twelve per SM, at most 32 splits), and the
@@ -64,16 +68,20 @@ cudaError_t pivoted_cholesky(const double* D, int64_t strideD, int n, double tol
 
 // The same factorisation of one matrix, blocked: a working copy of D in `work`
 // (pivoted_cholesky_work_doubles(n) doubles, device) is updated by a DMMA
-// product once per panel of 32 pivots; the pivots and the factor are those of
-// pivoted_cholesky up to rounding. info[0] = rank, info[1] = 1 when indefinite.
+// product once per panel of pivots; the pivots and the factor are those of
+// pivoted_cholesky up to rounding. Waits for the stream: *rank and *indefinite are
+// the host's, read from `mapped` (kPivotMapped bytes of page-locked host memory that
+// the kernel writes) or, when that is null, by a copy. n <= 22528.
+constexpr size_t kPivotMapped = 32;
 size_t pivoted_cholesky_work_doubles(int n);
-cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, int* info,
-                                     double* work, cudaStream_t stream);
+cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, double* work,
+                                     int64_t* rank, int* indefinite, cudaStream_t stream, void* mapped = nullptr);
 
-// Ct[i][mu] = Lc[i][mu] (i < info[2c], mu < n), zero padded to [opad][npad] per
-// cluster; sign[i] = 1 when sign is given.
+// Ct[i][mu] = Lc[i][mu] (i < info[2c], or < rank when info is null, mu < n), zero
+// padded to [opad][npad] per cluster; sign[i] = 1 when sign is given.
 cudaError_t factor_pad(const double* Lc, int64_t strideL, int64_t n, const int* info, double* Ct, int64_t strideCt,
-                       int64_t npad, int64_t opad, double* sign, int count, const int* active, cudaStream_t stream);
+                       int64_t npad, int64_t opad, double* sign, int count, const int* active, cudaStream_t stream,
+                       int64_t rank = 0);
 
 // Xt[(ql, i)][p] = sum_r B_{q0+ql}[p][r] Ct[i][r] for ql < qc, i < opad (one
 // cluster): the half-transform with the orbital index outermost, row stride npad.

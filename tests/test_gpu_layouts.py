@@ -14,6 +14,47 @@ pytestmark = pytest.mark.gpu
 EPS = 2.3e-16
 
 
+# column tiles of 32, 48, 64 and 80, one column more than each, several of them; odd n
+@pytest.mark.parametrize("columns", [1, 16, 17, 32, 33, 48, 49, 64, 65, 80, 81, 96, 97, 160, 161])
+@pytest.mark.parametrize("signed", [False, True])
+def test_exchange_of_every_column_tile(columns, signed):
+    import torch
+
+    n, n_aux = 129, 37
+    two_body = hydrogens(n, n_aux)
+    gen = torch.Generator().manual_seed(columns)
+    c = torch.randn((n, columns), dtype=torch.float64, generator=gen).cuda()
+    w = torch.randn(columns, dtype=torch.float64, generator=gen).cuda() if signed else None
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = two_body.orbital_tensor(eye, eye)
+    x = torch.einsum("quv,vi->qui", b, c)
+    expected = torch.einsum("qui,qvi->uv", x if w is None else x * w, x)
+    # two sums of n, then n_aux columns products: each errs by at most its length times eps times
+    # the sum of its absolute terms
+    ax = torch.einsum("quv,vi->qui", b.abs(), c.abs())
+    size = torch.einsum("qui,qvi->uv", ax if w is None else ax * w.abs(), ax)
+    got = two_body.exchange_factored(c, w)
+    assert float(((got - expected).abs() / ((2 * n + n_aux * columns) * EPS * size)).max()) < 1.0
+
+
+# one panel and several, rows of L in shared memory, ranks that end inside and at the end of a panel
+@pytest.mark.parametrize("n,rank", [(1, 1), (2, 1), (33, 33), (160, 40), (161, 161), (300, 70), (300, 95), (900, 64),
+                                    (900, 200)])
+def test_density_factor_across_panels(n, rank):
+    import torch
+
+    two_body = hydrogens(n, 3)
+    gen = torch.Generator().manual_seed(n + rank)
+    c = torch.randn((n, rank), dtype=torch.float64, generator=gen).cuda() / np.sqrt(n)
+    d = c @ c.T
+    f = two_body.context.density_factor_device(d, n)
+    assert rank <= f.shape[1] <= n
+    # a Cholesky factor reproduces each element to its length times eps of the diagonal's size, and the
+    # remainder it stops at is 1e-14 of the largest diagonal element
+    bound = ((rank + 2) * EPS + 1e-14) * float(d.diagonal().max()) * 4
+    assert float((f @ f.T - d).abs().max()) < bound
+
+
 # blocks of 64: one, a ragged one, several, with and without a remainder
 @pytest.mark.parametrize("n_aux", [1, 63, 64, 65, 127, 128, 130, 193, 256, 257, 321, 450])
 def test_the_fit_at_the_factors_block_edges(n_aux):
