@@ -172,17 +172,26 @@ __global__ void __launch_bounds__(kThreads) k_status(const double* __restrict__ 
     }
 }
 
-// Cyclic Jacobi eigendecomposition of a symmetric m x m matrix (m <= 9) held by
-// one thread: a becomes diagonal (eigenvalues), v holds the eigenvectors as columns.
-__device__ void jacobi_eigh(double (&a)[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS + 1],
-                            double (&v)[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS + 1], int m) {
-    for (int i = 0; i < m; ++i)
-        for (int j = 0; j < m; ++j) v[i][j] = i == j ? 1.0 : 0.0;
+// Cyclic Jacobi eigendecomposition of a symmetric m x m matrix (m <= 9) in shared
+// memory by one warp: a becomes diagonal (eigenvalues), v holds the eigenvectors as
+// columns. Lane k takes row (then column) k of a rotation, lane 16 + k row k of v;
+// one thread with the matrices in local memory took most of the DIIS kernel's 190 us.
+using DiisMatrix = double[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS + 1];
+__device__ void jacobi_eigh(DiisMatrix& a, DiisMatrix& v, int m) {
+    const int lane = threadIdx.x & 31, k = lane & 15;
+    const bool mine = k < m;
+    if (lane < m)
+        for (int j = 0; j < m; ++j) v[lane][j] = lane == j ? 1.0 : 0.0;
+    __syncwarp();
     for (int sweep = 0; sweep < 64; ++sweep) {
         double off = 0.0, diag = 0.0;
-        for (int i = 0; i < m; ++i) {
-            diag += a[i][i] * a[i][i];
-            for (int j = i + 1; j < m; ++j) off += a[i][j] * a[i][j];
+        if (lane < m) {
+            diag = a[lane][lane] * a[lane][lane];
+            for (int j = lane + 1; j < m; ++j) off += a[lane][j] * a[lane][j];
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            diag += __shfl_xor_sync(0xffffffffu, diag, o);
         }
         if (off <= 1e-32 * diag || off == 0.0) break;
         for (int p = 0; p < m - 1; ++p)
@@ -191,22 +200,21 @@ __device__ void jacobi_eigh(double (&a)[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS
                 if (apq == 0.0) continue;
                 const double theta = (a[q][q] - a[p][p]) / (2.0 * apq);
                 const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                const double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
-                for (int k = 0; k < m; ++k) {
-                    const double akp = a[k][p], akq = a[k][q];
-                    a[k][p] = cs * akp - sn * akq;
-                    a[k][q] = sn * akp + cs * akq;
+                const double cs = rsqrt(t * t + 1.0), sn = t * cs;
+                __syncwarp();
+                if (mine) {
+                    DiisMatrix& x = lane < 16 ? a : v;
+                    const double xp = x[k][p], xq = x[k][q];
+                    x[k][p] = cs * xp - sn * xq;
+                    x[k][q] = sn * xp + cs * xq;
                 }
-                for (int k = 0; k < m; ++k) {
-                    const double apk = a[p][k], aqk = a[q][k];
-                    a[p][k] = cs * apk - sn * aqk;
-                    a[q][k] = sn * apk + cs * aqk;
+                __syncwarp();
+                if (lane < m) {
+                    const double xp = a[p][k], xq = a[q][k];
+                    a[p][k] = cs * xp - sn * xq;
+                    a[q][k] = sn * xp + cs * xq;
                 }
-                for (int k = 0; k < m; ++k) {
-                    const double vkp = v[k][p], vkq = v[k][q];
-                    v[k][p] = cs * vkp - sn * vkq;
-                    v[k][q] = sn * vkp + cs * vkq;
-                }
+                __syncwarp();
             }
     }
 }
@@ -222,6 +230,7 @@ __global__ void __launch_bounds__(kThreads) k_diis(const double* __restrict__ F,
                                                    int diis) {
     __shared__ double red[33];
     __shared__ double coef[HF_BATCH_MAX_DIIS];
+    __shared__ DiisMatrix a, v;
     const int c = blockIdx.x;
     int* st = ints + c * kInts;
     const int64_t o = (int64_t)c * nn;
@@ -256,33 +265,32 @@ __global__ void __launch_bounds__(kThreads) k_diis(const double* __restrict__ F,
         if (threadIdx.x == 0) st[I_PUSHES] = pushes + 1;
         return;
     }
-    if (threadIdx.x == 0) {
-        double a[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS + 1], v[HF_BATCH_MAX_DIIS + 1][HF_BATCH_MAX_DIIS + 1];
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
         double scale = 0.0;
         for (int i = 0; i < cnt; ++i) scale = fmax(scale, O[i * HF_BATCH_MAX_DIIS + i]);
         const double inv = scale > 0.0 ? 1.0 / scale : 1.0;
-        for (int i = 0; i <= cnt; ++i)
+        if (lane <= cnt)
             for (int j = 0; j <= cnt; ++j) {
                 double x;
-                if (i < cnt && j < cnt) x = O[i * HF_BATCH_MAX_DIIS + j] * inv;
-                else if (i == cnt && j == cnt) x = 0.0;
+                if (lane < cnt && j < cnt) x = O[lane * HF_BATCH_MAX_DIIS + j] * inv;
+                else if (lane == cnt && j == cnt) x = 0.0;
                 else x = -1.0;
-                a[i][j] = x;
+                a[lane][j] = x;
             }
+        __syncwarp();
         jacobi_eigh(a, v, cnt + 1);
         double wmax = 0.0;
         for (int i = 0; i <= cnt; ++i) wmax = fmax(wmax, fabs(a[i][i]));
         // x = V diag(1/w) V^T r with r = (0, ..., 0, -1)
-        double sol[HF_BATCH_MAX_DIIS + 1];
-        for (int k = 0; k <= cnt; ++k) sol[k] = 0.0;
+        double sol = 0.0;
         for (int i = 0; i <= cnt; ++i) {
             const double w = a[i][i];
             if (!(fabs(w) > kNullSpaceTolerance * wmax)) continue;
-            const double proj = -v[cnt][i] / w;
-            for (int k = 0; k <= cnt; ++k) sol[k] += v[k][i] * proj;
+            if (lane <= cnt) sol += v[lane][i] * (-v[cnt][i] / w);
         }
-        for (int k = 0; k < cnt; ++k) coef[k] = sol[k];
-        st[I_PUSHES] = pushes + 1;
+        if (lane < cnt) coef[lane] = sol;
+        if (lane == 0) st[I_PUSHES] = pushes + 1;
     }
     __syncthreads();
     for (int64_t i = threadIdx.x; i < nn; i += blockDim.x) {
@@ -405,6 +413,161 @@ __global__ void __launch_bounds__(kThreads) k_pm_step(const double* __restrict__
     }
 }
 
+// The whole purification of one cluster per CTA: P and P^2 stay in shared memory
+// (n <= kPurifyMax), both products of a step on DMMA tiles, the steps and
+// coefficients of k_pm_step, ended as soon as the cluster has converged. As three
+// batched launches per step, all purify_steps of them in the graph, the launches
+// themselves were most of an iteration: 192 per batch and iteration, about 20 steps
+// of which do something. P, P^2 and P^3 are symmetric: only tiles touching the upper
+// triangle are computed, the lower one is their mirror image.
+constexpr int kPurifyMax = 112;
+constexpr int kPurifyTiles = 4;  // 16 x 8 tiles per warp: 56 upper ones at n = 112 over 16 warps
+static_assert(kThreads == 512, "k_purify deals its tiles to 16 warps");
+
+__host__ __device__ inline int purify_pad(int64_t m) { return (int)((m + 15) / 16 * 16); }
+inline size_t purify_smem(int64_t m) {
+    const size_t np = purify_pad(m);
+    return sizeof(double) * 2 * np * (np + 4);
+}
+
+// acc = the warp's upper tiles of A B^T, both np x np with pitch ld.
+__device__ __forceinline__ void upper_product(const double* A, const double* B, int np, int ld,
+                                              double (&acc)[kPurifyTiles][4]) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const int rb = np / 16, nt = np / 8;
+#pragma unroll
+    for (int u = 0; u < kPurifyTiles; ++u) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[u][x] = 0.0;
+        // tile t: row block r holds the column tiles 2r .. nt - 1
+        int t = warp + 16 * u, r = 0;
+        while (r < rb && t >= nt - 2 * r) {
+            t -= nt - 2 * r;
+            ++r;
+        }
+        if (r == rb) continue;  // the same for the whole warp
+        const double* a = A + (16 * r + gq) * ld + tq;
+        const double* b = B + (8 * (2 * r + t) + gq) * ld + tq;
+        double even[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k = 0; k < np; k += 16) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double (&c)[4] = h ? acc[u] : even;
+                const int kk = k + 8 * h;
+                asm volatile(
+                    "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                    "{%0,%1,%2,%3};\n"
+                    : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                    : "d"(a[kk]), "d"(a[kk + 8 * ld]), "d"(a[kk + 4]), "d"(a[kk + 8 * ld + 4]), "d"(b[kk]), "d"(b[kk + 4]));
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[u][x] += even[x];
+    }
+}
+
+// f(row, column, value) for the warp's elements on or above the diagonal.
+template <class Fn>
+__device__ __forceinline__ void upper_elements(int np, const double (&acc)[kPurifyTiles][4], Fn f) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const int rb = np / 16, nt = np / 8;
+#pragma unroll
+    for (int u = 0; u < kPurifyTiles; ++u) {
+        int t = warp + 16 * u, r = 0;
+        while (r < rb && t >= nt - 2 * r) {
+            t -= nt - 2 * r;
+            ++r;
+        }
+        if (r == rb) continue;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int i = 16 * r + gq + (x >> 1) * 8, j = 8 * (2 * r + t) + 2 * tq + (x & 1);
+            if (j >= i) f(i, j, acc[u][x]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_purify(double* __restrict__ Pg, int m, int steps, double tol,
+                                                     int* __restrict__ ints, int* __restrict__ act_pm) {
+    extern __shared__ double psm[];
+    __shared__ double red[33];
+    __shared__ double s_diag, s_inv, s_beta;
+    __shared__ int s_go;
+    const int c = blockIdx.x;
+    if (act_pm[c] == 0) return;
+    const int np = purify_pad(m), ld = np + 4;
+    double* P = psm;
+    double* P2 = psm + (size_t)np * ld;
+    double* g = Pg + (int64_t)c * m * m;
+    for (int e = threadIdx.x; e < np * np; e += blockDim.x) {
+        const int i = e / np, j = e - i * np;
+        // the upper triangle, mirrored
+        P[i * ld + j] = (i < m && j < m) ? g[(int64_t)min(i, j) * m + max(i, j)] : 0.0;
+    }
+    __syncthreads();
+    double acc[kPurifyTiles][4];
+    for (int step = 0; step < steps; ++step) {
+        upper_product(P, P, np, ld, acc);
+        double d1 = 0.0, d2 = 0.0, x3 = 0.0;
+        upper_elements(np, acc, [&](int i, int j, double p2) {
+            P2[i * ld + j] = p2;
+            P2[j * ld + i] = p2;
+            const double p = P[i * ld + j];
+            if (i == j) {
+                d1 += p - p2;
+                d2 += p2;
+                x3 += p2 * p;
+            } else {
+                x3 += 2.0 * p2 * p;
+            }
+        });
+        const double t1 = block_sum(d1, red);
+        const double tr2 = block_sum(d2, red);
+        const double tr3 = block_sum(x3, red);
+        if (threadIdx.x == 0) {
+            int* st = ints + c * kInts;
+            const double t2 = tr2 - tr3;
+            int go = 1;
+            if (st[I_CROSSED]) go = 0;
+            else if (t1 < tol) st[I_CROSSED] = 1;
+            double cc = 0.5;  // the McWeeny step when t1 is within rounding of zero
+            if (go) {
+                if (t1 > 0.0) cc = fmin(1.0, fmax(0.0, t2 / t1));
+                else if (!(fabs(t1) < tol)) {
+                    go = 0;  // eigenvalues left [0, 1]: no convergent purification
+                    st[I_STATE] = HF_SCF_PURIFICATION_FAILED;
+                }
+            }
+            if (go) {
+                st[I_PMSTEPS] += 1;
+                const double inv = 1.0 / (cc >= 0.5 ? cc : 1.0 - cc);
+                s_inv = inv;
+                s_diag = (1.0 + cc) * inv;
+                s_beta = cc >= 0.5 ? 0.0 : (1.0 - 2.0 * cc) * inv;
+            } else {
+                act_pm[c] = 0;
+            }
+            s_go = go;
+        }
+        __syncthreads();
+        if (!s_go) break;
+        // P' = P^2 ((1 + c) I - P) / d + beta P
+        upper_product(P2, P, np, ld, acc);
+        __syncthreads();  // every product has read P
+        const double inv = s_inv, diag = s_diag, beta = s_beta;
+        upper_elements(np, acc, [&](int i, int j, double p3) {
+            const double v = diag * P2[i * ld + j] - inv * p3 + beta * P[i * ld + j];
+            P[i * ld + j] = v;
+            P[j * ld + i] = v;
+        });
+        __syncthreads();
+    }
+    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
+        const int i = e / m, j = e - i * m;
+        g[e] = P[i * ld + j];
+    }
+}
+
 // Clusters whose purification has not ended after the captured steps fail.
 __global__ void k_pm_check(int count, const int* __restrict__ act_pm, int* __restrict__ ints,
                            int* __restrict__ act_next) {
@@ -497,7 +660,7 @@ struct hf_batch {
     double *ov = nullptr, *scal = nullptr, *pm_beta = nullptr;
     int *ints = nullptr, *info = nullptr, *act_grad = nullptr, *act_diis = nullptr, *act_next = nullptr,
         *act_pm = nullptr, *act_all = nullptr, *glob = nullptr;
-    std::vector<void*> allocations;
+    std::vector<void*> allocations, pooled;
     bool loaded = false;
     int64_t guess_rank = 0;
     int diis_alloc = HF_BATCH_MAX_DIIS;
@@ -518,8 +681,19 @@ int fail(hf_batch* b, int code, const std::string& msg) {
                         std::string(#call) + ": " + cudaGetErrorString(_e));                 \
     } while (0)
 
+// A batch's 35 blocks: small ones from the device's stream-ordered pool on the
+// batch's own stream (hf_batch_create waits for that stream before it returns), large
+// ones from cudaMalloc, as for the contexts. As 35 cudaMallocs, three batches took
+// 29 ms to create and 5 to destroy.
+constexpr size_t kPoolMaxBytes = (size_t)256 << 20;
 int balloc(hf_batch* b, void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 8);
+    const size_t size = bytes ? bytes : 8;
+    if (size < kPoolMaxBytes && cudaMallocAsync(p, size, b->own) == cudaSuccess) {
+        b->pooled.push_back(*p);
+        return HF_OK;
+    }
+    cudaGetLastError();
+    cudaError_t e = cudaMalloc(p, size);
     if (e != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
@@ -604,7 +778,10 @@ cudaError_t body(hf_batch* b, cudaStream_t s, const hf_batch_options& o, int* gr
     if ((e = gemm(b, fx, s)) != cudaSuccess) return e;
     if ((e = gemm(b, square(b, b->XT, b->T2, b->P, b->act_next, tile), s)) != cudaSuccess) return e;
     k_pm_init<<<cnt, kThreads, 0, s>>>(b->P, b->n, (double)b->nocc, b->act_next, b->act_pm, b->ints);
-    for (int step = 0; step < o.purify_steps; ++step) {
+    if (b->n <= kPurifyMax)
+        k_purify<<<cnt, kThreads, purify_smem(b->n), s>>>(b->P, (int)b->n, o.purify_steps, o.purify_tolerance, b->ints,
+                                                          b->act_pm);
+    for (int step = 0; b->n > kPurifyMax && step < o.purify_steps; ++step) {
         if ((e = gemm(b, square(b, b->P, b->P, b->P2, b->act_pm, tile), s)) != cudaSuccess) return e;
         k_pm_step<<<cnt, kThreads, 0, s>>>(b->P, b->P2, b->Y, b->n, b->pm_beta, b->ints, b->act_pm,
                                            o.purify_tolerance);
@@ -671,6 +848,12 @@ int hf_batch_create(hf_ctx* const* clusters, int count, int64_t n_occ, hf_batch*
     b->naux = v0.naux;
     b->npad = (int64_t)v0.nt * 64;
     cudaSetDevice(b->device);
+    if (cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        delete b;
+        return HF_ERR_CUDA;
+    }
+    b->stream = b->own;
     int s = HF_OK;
 #define HB_TAKE(ptr, elems)                                   \
     if ((s = take(b, &(ptr), (size_t)(elems))) != HF_OK) {    \
@@ -734,19 +917,18 @@ int hf_batch_create(hf_ctx* const* clusters, int count, int64_t n_occ, hf_batch*
         tab[c] = v.B;
     }
     std::vector<int> ones(count, 1);
-    // synchronous copies from pageable memory may return before their DMA lands; the
-    // device synchronisation orders them before any kernel on the batch's stream
-    if (cudaMemcpy(b->d_btab, tab.data(), sizeof(double*) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(b->act_all, ones.data(), sizeof(int) * count, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaDeviceSynchronize() != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking) != cudaSuccess) {
+    if (cudaMemcpyAsync(b->d_btab, tab.data(), sizeof(double*) * count, cudaMemcpyHostToDevice, b->own) != cudaSuccess ||
+        cudaMemcpyAsync(b->act_all, ones.data(), sizeof(int) * count, cudaMemcpyHostToDevice, b->own) != cudaSuccess ||
+        cudaStreamSynchronize(b->own) != cudaSuccess) {
         hf_batch_destroy(b);
         return HF_ERR_CUDA;
     }
     p.Btab = b->d_btab;
     b->plan = p;
-    b->stream = b->own;
-    if (jk_configure() != cudaSuccess) {
+    if (jk_configure() != cudaSuccess ||
+        cudaFuncSetAttribute(k_purify, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)purify_smem(kPurifyMax)) !=
+            cudaSuccess) {
+        cudaGetLastError();
         hf_batch_destroy(b);
         return HF_ERR_CUDA;
     }
@@ -758,7 +940,9 @@ int hf_batch_destroy(hf_batch* b) {
     if (!b) return HF_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
+    if (b->own) cudaStreamSynchronize(b->own);
     for (void* p : b->allocations) cudaFree(p);
+    for (void* p : b->pooled) cudaFreeAsync(p, b->own);
     if (b->own) cudaStreamDestroy(b->own);
     delete b;
     return HF_OK;

@@ -733,7 +733,7 @@ int hf_ctx_create(int device, hf_ctx** out) {
         return HF_ERR_ARG;
     }
     ctx->device = device;
-    if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&ctx->own, cudaStreamNonBlocking) != cudaSuccess) {
+    if (cudaSetDevice(device) != cudaSuccess || take_stream(device, &ctx->own) != cudaSuccess) {
         cudaGetLastError();
         delete ctx;
         return HF_ERR_CUDA;
@@ -786,7 +786,8 @@ int hf_ctx_destroy(hf_ctx* ctx) {
     flag_release(ctx->h_flag);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
-    if (ctx->own) cudaStreamDestroy(ctx->own);
+    if (ctx->own) cudaStreamSynchronize(ctx->own);
+    give_stream(ctx->device, ctx->own);
     delete ctx;
     return HF_OK;
 }

@@ -70,3 +70,19 @@ def test_the_fit_at_the_factors_block_edges(n_aux):
     condition = float(torch.linalg.cond(metric))
     bound = 8 * n_aux * EPS * condition * float(expected.abs().max())
     assert float((b - expected).abs().max()) < bound
+
+
+# the purification in one CTA (up to 112 functions) and in launches past it, n odd and at the edge
+@pytest.mark.parametrize("waters,basis", [(1, "sto-3g"), (1, "cc-pvdz"), (15, "sto-3g"), (16, "sto-3g"), (17, "sto-3g")])
+def test_batched_scf_at_the_purification_sizes(waters, basis):
+    from hafnium_b200.batch import solve_batch
+    from hafnium_b200.scf import DeviceHamiltonian, atomic_density_guess, solve_rhf
+
+    mols = [water_cluster(waters, s) for s in (1, 2)]
+    batch = solve_batch(mols, basis, setup_threads=2, retry_failed=False)
+    for mol, energy, state in zip(mols, batch.energies, batch.states):
+        ham = DeviceHamiltonian.build(mol, basis, "def2-universal-jkfit")
+        ref = solve_rhf(ham, guess=atomic_density_guess(mol, basis))
+        assert state == "converged"
+        # both stop at a commutator of 1e-6 or less, and the energy errs by its square
+        assert abs(energy - ref.energy) < 1e-8
