@@ -1429,8 +1429,7 @@ static int exchange_bf16(hf_ctx* ctx, const TcPlan& t, const double* Ct_tc, doub
     if (st != HF_OK) return st;
     double* Kp = ctx->d_tcwork;
     void* work = ctx->d_tcwork + kp_doubles;
-    HF_CU(cudaMemsetAsync(ctx->d_info + 2, 0, sizeof(int), ctx->stream));
-    const TcWait wait{ctx->d_info + 2, ctx->wait_ns, ctx->stall_next};
+    const TcWait wait{ctx->d_info + 2, ctx->wait_ns, ctx->stall_next, ctx->h_flag ? ctx->h_flag + kFlagBf16 : nullptr};
     ctx->stall_next = 0;
     cudaError_t e = exchange_build_bf16(t, ctx->d_bf16_b, Ct_tc, t.npad, dK, Kp, work, want - sizeof(double) * kp_doubles,
                                         wait, ctx->stream, ctx->n, sign);
@@ -1439,7 +1438,8 @@ static int exchange_bf16(hf_ctx* ctx, const TcPlan& t, const double* Ct_tc, doub
     int s = check_async(ctx, "split-BF16 exchange");
     if (s != HF_OK) return s;
     int flag = 0;
-    HF_CU(cudaMemcpy(&flag, ctx->d_info + 2, sizeof(int), cudaMemcpyDeviceToHost));
+    if (ctx->h_flag) flag = *(volatile int*)(ctx->h_flag + kFlagBf16);
+    else HF_CU(cudaMemcpy(&flag, ctx->d_info + 2, sizeof(int), cudaMemcpyDeviceToHost));
     if (flag) return fail(ctx, HF_ERR_TIMEOUT, "split-BF16 exchange: a pipeline wait ran out (code " +
                                                    std::to_string(flag) + ")");
     return HF_OK;

@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
 
 template <int EPT>
 cudaError_t launch_fused(const FusedArgs& a, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(k_coulomb_fused<EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_coulomb_fused<EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     // the grid's CTAs wait on one another: a cluster, or a cooperative grid
     cudaLaunchConfig_t c{};

@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "jk.cuh"
 #include "tc_exchange.cuh"
@@ -473,10 +474,11 @@ __global__ void __launch_bounds__(256) k_split_b_tiles(const double* __restrict_
     }
 }
 
-// C^T in FP64 ([opad][npad]) -> BF16 hi/lo.
+// C^T in FP64 ([opad][npad]) -> BF16 hi/lo. The build's first kernel: clears its error flag.
 __global__ void k_split_ct(const double* __restrict__ ct, int64_t count, __nv_bfloat16* __restrict__ h,
-                           __nv_bfloat16* __restrict__ l) {
+                           __nv_bfloat16* __restrict__ l, int* err) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e == 0) *err = 0;
     if (e >= count) return;
     const double x = ct[e];
     const __nv_bfloat16 hi = __double2bfloat16(x);
@@ -484,25 +486,29 @@ __global__ void k_split_ct(const double* __restrict__ ct, int64_t count, __nv_bf
     l[e] = __double2bfloat16(x - (double)__bfloat162float(hi));
 }
 
-// Kp[p][p'] += sum_s part[s][p][p'] over the elements of the stage-2 tiles that
-// touch the upper triangle ((p' / bn + 1) bn > (p / 128) 128), in a fixed order.
-__global__ void k_reduce_partials(const float* __restrict__ part, int splits, int64_t npad, int bn,
-                                  double* __restrict__ Kp) {
+// One chunk's partial sums in FP64, in split order, over mu <= nu < n (every such
+// element lies in a computed tile): added to the running sum Kp unless this is the
+// first chunk, and into K and its mirror image when it is the last (K is then exactly
+// symmetric, and the error flag goes to the host's copy of it, if there is one).
+__global__ void k_reduce_partials(const float* __restrict__ part, int splits, int64_t npad, int64_t n,
+                                  double* __restrict__ Kp, double* __restrict__ K, int first, int last,
+                                  const int* __restrict__ err, volatile int* host_err) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= npad * npad) return;
-    const int64_t row = e / npad, col = e % npad;
-    if ((col / bn + 1) * bn <= (row / BM) * BM) return;
-    double sum = 0.0;
-    for (int k = 0; k < splits; ++k) sum += (double)part[(int64_t)k * npad * npad + e];
-    Kp[e] += sum;
-}
-
-__global__ void k_symmetrize_upper128(const double* __restrict__ Kp, int64_t ldk, int64_t n, double* __restrict__ K) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e == 0 && last && host_err) *host_err = *err;
     if (e >= n * n) return;
     const int64_t mu = e / n, nu = e % n;
-    // element-level mirror: K is exactly symmetric (every mu <= nu lies in a computed tile)
-    K[e] = mu <= nu ? Kp[mu * ldk + nu] : Kp[nu * ldk + mu];
+    if (mu > nu) return;
+    const int64_t at = mu * npad + nu;
+    double sum = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) sum += (double)part[(int64_t)k * npad * npad + at];
+    if (!first) sum += Kp[at];
+    if (!last) {
+        Kp[at] = sum;
+        return;
+    }
+    K[e] = sum;
+    K[nu * n + mu] = sum;
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -541,11 +547,28 @@ int sm_count() {
     return sms;
 }
 
+// The kernel's shared memory limit, set once per device: set before every launch to
+// that launch's size, it changed twice per build, and each change held up the next
+// launch in the driver.
+cudaError_t tc_configure() {
+    static std::mutex mutex;
+    static bool done[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (done[dev]) return cudaSuccess;
+    e = cudaFuncSetAttribute(k_tc_split3, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    done[dev] = e == cudaSuccess;
+    return e;
+}
+
 // One persistent CTA per SM (at most one per work item).
 cudaError_t launch_tc(const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, const CUtensorMap& bl,
                       const TcParams& P, cudaStream_t stream) {
     const size_t smem = smem_for(P.bn, P.stages);
-    cudaError_t e = cudaFuncSetAttribute(k_tc_split3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = tc_configure();
     if (e != cudaSuccess) return e;
     if (P.items < 1) return cudaSuccess;
     const int grid = std::min(P.items, sm_count());
@@ -637,8 +660,7 @@ cudaError_t exchange_build_bf16(const TcPlan& t, const void* bf16_b, const doubl
     int qchunk = (int)std::min<size_t>((work_bytes - head) / per_q, (size_t)t.naux);
     if (qchunk < 1) return cudaErrorInvalidValue;
     const int64_t cnt = (int64_t)t.opad * npad;
-    k_split_ct<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(Ct_fp64, cnt, cth, ctl);
-    cudaMemsetAsync(Kp, 0, sizeof(double) * npad * npad, stream);
+    k_split_ct<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(Ct_fp64, cnt, cth, ctl, wait.err);
     CUtensorMap mCh, mCl;
     if (!make_map(&mCh, cth, t.opad, npad, t.bn1) || !make_map(&mCl, ctl, t.opad, npad, t.bn1))
         return cudaErrorInvalidValue;
@@ -706,9 +728,9 @@ cudaError_t exchange_build_bf16(const TcPlan& t, const void* bf16_b, const doubl
         Q.stall = 0;
         e = launch_tc(mXh, mXl, mXh2, mXl2, Q, stream);
         if (e != cudaSuccess) return e;
-        k_reduce_partials<<<(unsigned)((npad * npad + 255) / 256), 256, 0, stream>>>(kpart, Q.splits, npad, bn2, Kp);
+        k_reduce_partials<<<(unsigned)((n * n + 255) / 256), 256, 0, stream>>>(
+            kpart, Q.splits, npad, n, Kp, K, q0 == 0, q0 + qc >= t.naux, wait.err, wait.host_err);
     }
-    k_symmetrize_upper128<<<(unsigned)((n * n + 255) / 256), 256, 0, stream>>>(Kp, npad, n, K);
     return cudaGetLastError();
 }
 

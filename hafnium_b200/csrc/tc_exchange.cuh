@@ -24,13 +24,15 @@ size_t tc_b_bytes(int64_t n, int naux);
 size_t tc_partial_bytes(int64_t npad);
 // Fill the BF16 hi/lo copies ([naux][npad][npad] each, hi first) from the FP64 tiles.
 cudaError_t tc_split_b(const JkPlan& p, int64_t npad, void* bf16_b, cudaStream_t stream);
-// The pipeline's bounded waits: err (device int, zeroed by the caller) is set to
-// 1 when a wait runs out after wait_ns; stall makes the first stage-1 launch
+// The pipeline's bounded waits: err (device int, zeroed by the build) is set to 1
+// when a wait runs out after wait_ns, and copied to host_err (page-locked, may be
+// null) at the build's end; stall makes the first stage-1 launch
 // wait once on a barrier that nothing completes (a self-test of that path).
 struct TcWait {
     int* err;
     uint64_t wait_ns;
     int stall;
+    int* host_err;
 };
 
 // K = sum_q (B_q C) diag(sign) (B_q C)^T with split-BF16 products; Ct_fp64 is
