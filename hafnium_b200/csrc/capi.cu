@@ -73,8 +73,9 @@ struct hf_ctx {
     double* d_metric = nullptr;  // N x N internal order
     double* d_B = nullptr;       // N x ntiles*4096
     // scratch
-    double* d_work = nullptr;
+    double* d_work = nullptr;  // J build
     size_t work_bytes = 0;
+    PacketSpace packets;  // ... as the one-pass build left it
     double* d_io = nullptr;  // host-transfer staging: 2 n x n
     size_t io_bytes = 0;
     double* d_kscratch = nullptr;  // K build: Kp | X | Xs
@@ -455,6 +456,7 @@ void trelease(hf_ctx* ctx, T*& p) {
 
 int ensure_work(hf_ctx* ctx, size_t bytes) {
     if (ctx->work_bytes >= bytes) return HF_OK;
+    ctx->packets.next = 0;
     big_release(ctx, ctx->d_work, ctx->work_bytes);
     return big_alloc(ctx, (void**)&ctx->d_work, bytes, &ctx->work_bytes);
 }
@@ -1312,9 +1314,10 @@ static size_t coulomb_doubles(const hf_ctx* ctx, const JkPlan& p, bool* fused) {
 }
 
 static int coulomb_run(hf_ctx* ctx, const JkPlan& p, bool fused, const double* D, double* J, double* work,
-                       double* host_out, const char* what) {
+                       PacketSpace& held, double* host_out, const char* what) {
     const size_t bytes = sizeof(double) * (size_t)p.n * p.n;
     if (!fused) {
+        held.next = 0;
         HF_CU(coulomb_build(p, D, J, work, ctx->stream));
         ctx->stats.kernel_launches += 4;
         if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1322,7 +1325,7 @@ static int coulomb_run(hf_ctx* ctx, const JkPlan& p, bool fused, const double* D
     }
     std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
     if (coulomb_fused_cooperative(p)) lock.lock();
-    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, ctx->h_flag, ctx->wait_ns, ctx->stream));
+    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, ctx->wait_ns, ctx->stream));
     ++ctx->stats.kernel_launches;
     if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     const int s = check_async(ctx, what);
@@ -1342,11 +1345,7 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
     int s;
     bool fused = false;
     const size_t need = coulomb_doubles(ctx, p, &fused);
-    if (ctx->work_bytes < sizeof(double) * need) {
-        if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
-        // the one-pass build tells its packets from what the block held before by their tags
-        HF_CU(cudaMemsetAsync(ctx->d_work, 0, ctx->work_bytes, ctx->stream));
-    }
+    if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
     const double* dD = D;
     double* dJ = J;
     if (!on_device) {
@@ -1356,7 +1355,7 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
         dJ = ctx->d_io + nn;
     }
     time_begin(ctx);
-    s = coulomb_run(ctx, p, fused, dD, dJ, ctx->d_work, on_device ? nullptr : J, "hf_coulomb");
+    s = coulomb_run(ctx, p, fused, dD, dJ, ctx->d_work, ctx->packets, on_device ? nullptr : J, "hf_coulomb");
     ctx->stats.ms_coulomb = time_end(ctx);
     return s;
 }
@@ -2356,6 +2355,7 @@ static __device__ __align__(256) double g_coulomb_scratch[kStaticScratchDoubles]
 constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mutex;
 double* g_scratch_ptr[kMaxDevices] = {};
+PacketSpace g_scratch_packets[kMaxDevices];  // as shared as the array: the caller serialises the calls
 
 // Device address of g_coulomb_scratch on `device` (current), resolved once.
 int static_scratch(hf_ctx* ctx, double** out) {
@@ -2390,5 +2390,6 @@ extern "C" int hf_coulomb_static(hf_ctx* ctx, const double* density, double* cou
     bool fused = false;
     if (coulomb_doubles(ctx, p, &fused) > (size_t)kStaticScratchDoubles)
         return fail(ctx, HF_ERR_ARG, "scratch size exceeded");
-    return coulomb_run(ctx, p, fused, density, coulomb, scratch, nullptr, "hf_coulomb_static");
+    return coulomb_run(ctx, p, fused, density, coulomb, scratch, g_scratch_packets[ctx->device], nullptr,
+                       "hf_coulomb_static");
 }

@@ -18,9 +18,12 @@
 //     5 us of HBM traffic) beside the 200 KB in flight.
 //   * A publishing warp adds the workers' partial sums and sends them to the
 //     group through global memory; collecting warps add the group's partials in
-//     CTA order. A packet is 16 bytes, {low, tag, high, tag}: each 8-byte half
-//     carries its own tag, so a packet is complete when both tags match and no
-//     fence or counter is needed. Tags are unique per launch and row block.
+//     CTA order. A packet is 16 bytes, {low, tag, high, tag} (the layout of NCCL's
+//     low-latency protocol): each 8-byte half carries its own tag, so a packet is
+//     complete when both tags match and no fence or counter is needed. A tag is
+//     used once between two zeroings of the workspace, which is zeroed whenever
+//     something else may lie in it (PacketSpace): no value of another kernel's
+//     data can pass for a packet.
 //     Groups of more than 32 CTAs send to an owner of the row that hands out the
 //     sum (two hops, but 2 E packets instead of E^2 reads of them).
 //   * The CTAs wait on one another: a small grid is one thread-block cluster, a
@@ -727,20 +730,9 @@ size_t packet_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql
 size_t sum_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b; }
 size_t jpart_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ge * a.pp; }
 
-// Tags count up within [kTagBase, kTagBase + kTagCount): as integers, floats or halves of doubles
-// these words do not occur in the data that other kernels leave in the same memory (small counts
-// did), and a tag comes back only after 2^28 row blocks.
-constexpr uint32_t kTagBase = 0x80000000u, kTagCount = 1u << 28;
-std::atomic<uint32_t> g_tag{0};
-
-// The first of `count` consecutive tags.
-uint32_t take_tags(uint32_t count) {
-    uint32_t at = g_tag.load(), from;
-    do {
-        from = at + count <= kTagCount ? at : 0;
-    } while (!g_tag.compare_exchange_weak(at, from + count));
-    return kTagBase + from;
-}
+size_t flag_bytes(const FusedArgs& a) { return ((size_t)8 * a.gq * a.ge + 15) / 16 * 16 + 16; }  // and the stop word
+// what a build tells from older contents by its tags, at the front of the workspace
+size_t tagged_bytes(const FusedArgs& a) { return packet_bytes(a) + sum_bytes(a) + flag_bytes(a); }
 
 int device_sms() {
     static std::atomic<int> sms[64];
@@ -759,7 +751,7 @@ int device_sms() {
 size_t coulomb_fused_work_doubles(const JkPlan& p) {
     const FusedShape f = plan_coulomb(p, device_sms());
     if (!f.ept) return 0;
-    return (packet_bytes(f.a) + sum_bytes(f.a) + jpart_bytes(f.a) + 8 * (size_t)f.a.gq * f.a.ge) / 8 + 4;
+    return (tagged_bytes(f.a) + jpart_bytes(f.a)) / 8 + 2;
 }
 
 bool coulomb_fused_cooperative(const JkPlan& p) {
@@ -772,8 +764,8 @@ std::mutex& cooperative_mutex(int device) {
     return mutexes[device >= 0 && device < 64 ? device : 0];
 }
 
-cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work, int* err,
-                                uint64_t wait_ns, cudaStream_t stream) {
+cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
+                                PacketSpace& held, int* err, uint64_t wait_ns, cudaStream_t stream) {
     const FusedShape f = plan_coulomb(p, device_sms());
     if (!f.ept) return cudaErrorInvalidValue;
     FusedArgs a = f.a;
@@ -787,10 +779,19 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     a.J = J;
     a.packets = reinterpret_cast<uint4*>((reinterpret_cast<uintptr_t>(work) + 15) & ~uintptr_t(15));
     a.sums = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.packets) + packet_bytes(a));
-    a.jpart = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(a.sums) + sum_bytes(a));
-    a.jflag = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(a.jpart) + jpart_bytes(a));
+    a.jflag = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(a.sums) + sum_bytes(a));
     a.stop = reinterpret_cast<uint32_t*>(a.jflag + (size_t)a.gq * a.ge);
-    a.tag = take_tags((uint32_t)a.blocks + 1);
+    a.jpart = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(a.packets) + tagged_bytes(a));
+    // no word of the tagged part holds a tag of this build: it holds smaller tags of builds of this shape, or zeros
+    const uint32_t tags = (uint32_t)a.blocks + 1;
+    if (held.next == 0 || held.n != p.n || held.naux != p.naux || held.next > UINT32_MAX - tags) {
+        held.next = 0;
+        const cudaError_t e = cudaMemsetAsync(a.packets, 0, tagged_bytes(a), stream);
+        if (e != cudaSuccess) return e;
+        held = PacketSpace{p.n, p.naux, 1};
+    }
+    a.tag = held.next;
+    held.next += tags;
     a.err = err;
     a.wait_ns = wait_ns;
     switch (f.ept) {

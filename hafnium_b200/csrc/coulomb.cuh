@@ -11,9 +11,18 @@ namespace hf {
 
 // The Coulomb build of one cluster in one pass over B (coulomb.cu). Applies when
 // coulomb_fused_work_doubles(p) > 0 (the slices of J and D fit the registers of
-// one CTA per SM: n up to about 1100); work holds that many doubles, zeroed once
-// when it is allocated.
+// one CTA per SM: n up to about 1100); work holds that many doubles.
 size_t coulomb_fused_work_doubles(const JkPlan& p);
+
+// What a workspace of the one-pass build holds: packets of builds of this shape with
+// tags below `next`, or, with next == 0, anything (a build of another shape, or with
+// next == 0, zeroes the packets first). Whoever allocates the workspace or writes
+// something else to it sets next to 0.
+struct PacketSpace {
+    int64_t n = 0;
+    int naux = 0;
+    uint32_t next = 0;
+};
 
 // J = scale * sum_q (B_q . D) B_q, J full n x n. The grid's CTAs wait on one another,
 // bounded by wait_ns; past it *err (device-visible, 0 before) becomes 1 and J is
@@ -21,8 +30,8 @@ size_t coulomb_fused_work_doubles(const JkPlan& p);
 // (coulomb_fused_cooperative): hold cooperative_mutex(device) from its launch to its
 // completion, since two such grids in flight could each hold SMs that the other waits for.
 bool coulomb_fused_cooperative(const JkPlan& p);
-cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work, int* err,
-                                uint64_t wait_ns, cudaStream_t stream);
+cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
+                                PacketSpace& held, int* err, uint64_t wait_ns, cudaStream_t stream);
 
 std::mutex& cooperative_mutex(int device);
 

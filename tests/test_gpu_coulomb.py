@@ -11,14 +11,17 @@ from hafnium_b200.jk import B200DensityFittedCoulombExchange
 pytestmark = pytest.mark.gpu
 
 
-def hydrogens(n, n_aux):
-    """A builder with exactly n orbital and n_aux auxiliary functions: s shells on a jittered grid."""
+def hydrogen_tables(n, n_aux):
+    """Tables of exactly n orbital and n_aux auxiliary functions: s shells on a jittered grid."""
     rng = np.random.default_rng(n)
     side = int(np.ceil(max(n, n_aux) ** (1 / 3)))
     grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
     at = 1.4 * grid + rng.uniform(-0.2, 0.2, size=grid.shape)
-    return B200DensityFittedCoulombExchange.from_tables(ShellTable.build("sto-3g", ["H"] * n, at[:n]),
-                                                        ShellTable.build("sto-3g", ["H"] * n_aux, at[:n_aux]))
+    return (ShellTable.build("sto-3g", ["H"] * n, at[:n]), ShellTable.build("sto-3g", ["H"] * n_aux, at[:n_aux]))
+
+
+def hydrogens(n, n_aux):
+    return B200DensityFittedCoulombExchange.from_tables(*hydrogen_tables(n, n_aux))
 
 
 # one piece, odd counts, the tile edges, each form of the exchange between CTAs (none, by lanes, by
@@ -73,5 +76,37 @@ for tag in ("water", "h2o2_s0", "h2o4_s1"):
         d = d + d.T
         first, second = two_body.coulomb(d), two_body.coulomb(d)
         assert torch.equal(first, second), (tag, rep, float((first - second).abs().max()))
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("static", [False, True])
+def test_a_scratch_that_holds_negative_zeros(static):
+    """The weighted density of the two-pass build may hold -0.0, whose upper half is 0x80000000. The first
+    one-pass builds of a process, in the memory that such a density was left in, give the contraction of B."""
+    import subprocess
+    import sys
+
+    code = f"""
+import torch
+from hafnium_b200 import _lib
+from tests.test_gpu_coulomb import hydrogen_tables
+context = _lib.Context()
+for n, n_aux in ((1410, 40), (24, 113), (1410, 40), (129, 300), (390, 150)):
+    context.upload(*hydrogen_tables(n, n_aux))
+    context.build()
+    if n > 1100:
+        d = torch.full((n, n), -0.0, dtype=torch.float64, device="cuda")
+    else:
+        c = torch.randn((n, 5), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+        d = c @ c.T
+    got = torch.empty_like(d)
+    (context.coulomb_static_device if {static} else context.coulomb_device)(d, got)
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = context.mo_fitted_tensor(eye, eye)
+    expected = torch.einsum("quv,q->uv", b, torch.einsum("quv,uv->q", b, d))
+    # two sums of n^2 and n_aux rounded products in another order
+    size = torch.einsum("quv,q->uv", b.abs(), torch.einsum("quv,uv->q", b.abs(), d.abs()))
+    assert bool(((got - expected).abs() <= 2.3e-16 * (n * n + n_aux) * size).all()), (n, n_aux)
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
