@@ -1048,6 +1048,8 @@ static void chunk_tasks(const hf_ctx* ctx, int row0, int row1, std::vector<PairT
     chunk_tasks_from(ctx, screen_pairs(ctx), row0, row1, tasks, max_npp);
 }
 
+constexpr const char* kTooManyPrimitives = "a shell pair has too many primitive pairs for the three-centre kernels";
+
 // Three-centre integrals of tile rows [row0, row1) into T ([cols][naux]).
 static int three_center_chunk(hf_ctx* ctx, int row0, int row1, double* T, PairTask* d_tasks, size_t task_cap) {
     std::vector<PairTask> tasks[3][3];
@@ -1061,6 +1063,10 @@ static int three_center_chunk(hf_ctx* ctx, int row0, int row1, double* T, PairTa
             most = std::max(most, tasks[la][lb].size() * (size_t)pair_data_stride(la, lb, max_npp[la][lb]));
         }
     if (pairs > task_cap) return fail(ctx, HF_ERR_STATE, "task buffer too small");
+    for (int la = 0; la <= 2; ++la)
+        for (int lb = la; lb <= 2; ++lb)
+            if (!tasks[la][lb].empty() && !three_center_fits(la, lb, max_npp[la][lb], ctx->aux_count))
+                return fail(ctx, HF_ERR_ARG, kTooManyPrimitives);
     double* data = nullptr;
     int* npps = nullptr;
     if (talloc(ctx, (void**)&data, sizeof(double) * most) || talloc(ctx, (void**)&npps, sizeof(int) * (pairs + 1))) {
@@ -1198,6 +1204,12 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
                 all_tasks.insert(all_tasks.end(), v.begin(), v.end());
             }
     }
+    for (const auto& chunk : launches)
+        for (const Launch& l : chunk)
+            if (!three_center_fits(l.la, l.lb, l.max_npp, ctx->aux_count)) {
+                trelease(ctx, Linv);
+                return fail(ctx, HF_ERR_ARG, kTooManyPrimitives);
+            }
     // one chunk's pair data: every class of the largest chunk side by side
     std::vector<size_t> data_at(6 * chunks.size() + 1, 0);
     size_t data_doubles = 0;
@@ -1252,7 +1264,9 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
                                  ctx->d_coefs, data_of(i), br.next());
             ++ctx->stats.kernel_launches;
         }
-        if (e == cudaSuccess) e = br.join();
+        // joined also after a failed launch: the buffers are freed in the order of the context's stream
+        cudaError_t je = br.join();
+        if (e == cudaSuccess) e = je;
         if (e == cudaSuccess) e = br.fork();
         for (size_t i = 0; i < launches[c].size() && e == cudaSuccess; ++i) {
             const Launch& l = launches[c][i];
@@ -1261,7 +1275,8 @@ int hf_build_fitted_tensor(hf_ctx* ctx) {
                                     data_of(i), T, br);
             ctx->stats.kernel_launches += 5;
         }
-        if (e == cudaSuccess) e = br.join();
+        je = br.join();
+        if (e == cudaSuccess) e = je;
         cudaEventRecord(ev[3 * c + 1], ctx->stream);
         if (e == cudaSuccess)
             e = apply_inverse_factor(Linv, N, N, T, N, ncols, ctx->d_B + t0 * 4096, ldb, ctx->stream, q_begin, q_end);

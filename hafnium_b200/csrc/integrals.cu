@@ -446,6 +446,28 @@ cudaError_t launch_pair_data(int la, int lb, const PairTask* tasks, int ntasks, 
     return e;
 }
 
+namespace {
+// Dynamic shared memory up to which no kernel here needs its limit raised: the static
+// tables count against the 48 KB default too.
+constexpr size_t kPlainShared = 40 * 1024;
+
+// The most dynamic shared memory a launch of `kernel` may have: the device's limit less
+// the kernel's static part.
+template <class Kernel>
+bool shared_fits(Kernel* kernel, size_t smem) {
+    if (smem <= kPlainShared) return true;
+    int device = 0, most = 0;
+    cudaFuncAttributes at{};
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
+        cudaFuncGetAttributes(&at, kernel) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return smem + at.sharedSizeBytes <= (size_t)most;
+}
+}  // namespace
+
 int64_t pair_data_stride(int la, int lb, int max_npp) {
     int64_t stride = 0;
 #define HF_STRIDE(LA, LB) \
@@ -746,6 +768,30 @@ cudaError_t launch_three_center(int la, int lb, const PairTask* tasks, int ntask
 #undef HF_3C_P
 #undef HF_3C
     return e;
+}
+
+template <int LA, int LB, int LP>
+static bool three_center_one_fits(int max_npp) {
+    return shared_fits(k_three_center<LA, LB, LP>,
+                       sizeof(double) * ((size_t)max_npp * PairLayout<LA, LB>::STRIDE + ThreeCenterShape<LA, LB, LP>::R_DOUBLES));
+}
+
+bool three_center_fits(int la, int lb, int max_npp, const int* count) {
+    bool fits = true;
+#define HF_3CF(LA, LB, LP) (count[LP] == 0 || three_center_one_fits<LA, LB, LP>(max_npp))
+#define HF_3CF_P(LA, LB)                                                                                       \
+    if (la == LA && lb == LB)                                                                                  \
+        fits = shared_fits(k_pair_data<LA, LB>, sizeof(double) * (size_t)max_npp * PairLayout<LA, LB>::STRIDE) && \
+               HF_3CF(LA, LB, 0) && HF_3CF(LA, LB, 1) && HF_3CF(LA, LB, 2) && HF_3CF(LA, LB, 3) && HF_3CF(LA, LB, 4);
+    HF_3CF_P(0, 0)
+    HF_3CF_P(0, 1)
+    HF_3CF_P(0, 2)
+    HF_3CF_P(1, 1)
+    HF_3CF_P(1, 2)
+    HF_3CF_P(2, 2)
+#undef HF_3CF_P
+#undef HF_3CF
+    return fits;
 }
 
 // ---------------------------------------------------------- S, T and V

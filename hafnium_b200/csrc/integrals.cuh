@@ -130,6 +130,11 @@ cudaError_t launch_pair_data(int la, int lb, const PairTask* tasks, int ntasks, 
                              const double* exps, const double* coefs, PairData pd, cudaStream_t stream);
 int64_t pair_data_stride(int la, int lb, int max_npp);
 
+// Whether the shared memory of launch_pair_data and launch_three_center holds pairs of
+// max_npp primitive pairs: asked before the first launch of a build, so that none fails
+// with others in flight.
+bool three_center_fits(int la, int lb, int max_npp, const int* aux_count);
+
 // S, T (kinetic) or V (attraction to point charges) over all ordered shell pairs
 // of class (la, lb) into out[n][n] (AO order). kind: 0 S, 1 T, 2 V.
 cudaError_t launch_one_electron(int kind, int la, int lb, const int2* tasks, int ntasks, const DevShell* orb,

@@ -9,6 +9,8 @@ import numpy as np
 import pytest
 
 from hafnium_b200 import _lib
+from hafnium_b200.basis import ShellTable
+from hafnium_b200.errors import InputError
 from oracle import dfrhf, kernels
 from tests.helpers import molecule, tables, water_sto3g_pyscf_geometry
 
@@ -89,3 +91,36 @@ def test_four_center_matches_oracle():
     ctx = _lib.Context(0)
     ctx.upload(orb)
     np.testing.assert_allclose(ctx.four_center(), dfrhf.eri_exact(orb), atol=ORACLE_TOL, rtol=0)
+
+
+def contracted(n_prim, centers):
+    """An s shell of three primitives and a d shell of ``n_prim`` on every centre."""
+    centers = np.asarray(centers, dtype=np.float64)
+    n = len(centers)
+    exps = [np.array([0.4, 1.7, 6.0]), 0.5 * 2.2 ** np.arange(n_prim)]
+    coefs = [np.array([0.5, 0.4, 0.2]), np.linspace(0.6, 0.1, n_prim)]
+    return ShellTable(np.tile([0, 2], n), np.repeat(centers, 2, axis=0),
+                      np.concatenate([[0], np.cumsum(np.tile([3, n_prim], n))]).astype(np.int64),
+                      np.tile(np.concatenate(exps), n), np.tile(np.concatenate(coefs), n),
+                      np.ones(2 * n, dtype=np.int64), np.repeat(np.arange(n), 2))
+
+
+# d-d pairs of 25 primitive pairs are the most that the three-centre kernels' shared memory holds
+@pytest.mark.parametrize("n_prim,fits", [(5, True), (6, False)])
+def test_shell_pairs_at_the_shared_memory_limit(n_prim, fits):
+    mol = molecule("water")
+    water_orb, aux = tables(mol)
+    orb = contracted(n_prim, mol.positions)
+    ctx = context_for(orb, aux)
+    if fits:
+        np.testing.assert_allclose(ctx.three_center(), dfrhf.three_center(aux, orb), atol=ORACLE_TOL, rtol=0)
+        ctx.build()
+        return
+    for _ in range(2):
+        with pytest.raises(InputError, match="too many primitive pairs"):
+            ctx.build()
+        with pytest.raises(InputError, match="too many primitive pairs"):
+            ctx.three_center()
+    ctx.upload(water_orb, aux)
+    ctx.build()
+    np.testing.assert_allclose(ctx.three_center(), dfrhf.three_center(aux, water_orb), atol=ORACLE_TOL, rtol=0)
