@@ -494,13 +494,8 @@ static cudaError_t three_center_grad_one(const PairTask* tasks, int ntasks, int 
     if (ntasks == 0 || nalist == 0) return cudaSuccess;
     using SH = GradCenterShape<LA, LB, LP>;
     const size_t smem = sizeof(double) * (size_t)SH::R_DOUBLES;
-    // the attribute covers the dynamic part; the static tables count against
-    // the 48 KB default too
-    if (smem > 32 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_three_center_grad<LA, LB, LP>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared((const void*)k_three_center_grad<LA, LB, LP>, smem);
+    if (e != cudaSuccess) return e;
     const int share = triple_share(ntasks, nalist, SH::SPW, kGradCenterThreads / 32, max_npp, SH::TPR, INT32_MAX);
     const int per_cta = kGradCenterThreads / 32 * (SH::SPW / share);
     dim3 grid(ntasks, (nalist + per_cta - 1) / per_cta);
@@ -538,11 +533,8 @@ static cudaError_t grad_pair_data_one(const PairTask* tasks, int ntasks, int max
     if (ntasks == 0) return cudaSuccess;
     const size_t smem = sizeof(double) * (size_t)max_npp * GradPairLayout<LA, LB>::STRIDE;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_grad_pair_data<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared((const void*)k_grad_pair_data<LA, LB>, smem);
+    if (e != cudaSuccess) return e;
     k_grad_pair_data<LA, LB><<<ntasks, kGradThreads, smem, stream>>>(tasks, orb, exps, coefs, D, n, pd.offsets,
                                                                      pd.data, pd.npps);
     return cudaGetLastError();

@@ -9,7 +9,9 @@
 // applied to the bra pair's Hermite coefficients once per primitive pair instead
 // of to every output block (cartesian.rs:93-110, two_electron.rs:1028-1060).
 #include <cmath>
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "integrals.cuh"
@@ -405,6 +407,30 @@ __device__ int pair_prologue(const DevShell& A, const DevShell& B, const double*
     return nk;
 }
 
+cudaError_t allow_shared(const void* kernel, size_t smem) {
+    if (smem <= kPlainShared) return cudaSuccess;
+    static std::mutex mutex;
+    static std::map<std::pair<const void*, int>, size_t> limits;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    size_t& most = limits[{kernel, device}];
+    if (most == 0) {
+        int bytes = 0;
+        cudaFuncAttributes at{};
+        e = cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, kernel);
+        if (e == cudaSuccess) {
+            bytes -= (int)at.sharedSizeBytes;
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        }
+        if (e != cudaSuccess) return e;
+        most = (size_t)bytes;
+    }
+    return smem <= most ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 // The pair data of pair_prologue, built once per shell pair into global memory (stride doubles per
 // task) for every auxiliary class and slab: a CTA per (pair, slab) that builds it itself spends most
 // of its time on it for the high classes, whose pairs have few primitives and whose slabs are many.
@@ -427,10 +453,8 @@ template <int LA, int LB>
 static cudaError_t pair_data_one(const PairTask* tasks, int ntasks, int max_npp, const DevShell* orb,
                                  const double* exps, const double* coefs, PairData pd, cudaStream_t stream) {
     const size_t smem = sizeof(double) * (size_t)max_npp * PairLayout<LA, LB>::STRIDE;
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_pair_data<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared((const void*)k_pair_data<LA, LB>, smem);
+    if (e != cudaSuccess) return e;
     k_pair_data<LA, LB><<<ntasks, 128, smem, stream>>>(tasks, orb, exps, coefs, pd.data, pd.stride, pd.npps);
     return cudaGetLastError();
 }
@@ -445,28 +469,6 @@ cudaError_t launch_pair_data(int la, int lb, const PairTask* tasks, int ntasks, 
 #undef HF_PD
     return e;
 }
-
-namespace {
-// Dynamic shared memory up to which no kernel here needs its limit raised: the static
-// tables count against the 48 KB default too.
-constexpr size_t kPlainShared = 40 * 1024;
-
-// The most dynamic shared memory a launch of `kernel` may have: the device's limit less
-// the kernel's static part.
-template <class Kernel>
-bool shared_fits(Kernel* kernel, size_t smem) {
-    if (smem <= kPlainShared) return true;
-    int device = 0, most = 0;
-    cudaFuncAttributes at{};
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
-        cudaFuncGetAttributes(&at, kernel) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return smem + at.sharedSizeBytes <= (size_t)most;
-}
-}  // namespace
 
 int64_t pair_data_stride(int la, int lb, int max_npp) {
     int64_t stride = 0;
@@ -734,13 +736,8 @@ static cudaError_t three_center_one(const PairTask* tasks, int ntasks, int max_n
     using SH = ThreeCenterShape<LA, LB, LP>;
     const int r_offset = max_npp * PairLayout<LA, LB>::STRIDE;
     const size_t smem = sizeof(double) * ((size_t)r_offset + SH::R_DOUBLES);
-    // the attribute covers the dynamic part; the static tables count against
-    // the 48 KB default too
-    if (smem > 40 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_three_center<LA, LB, LP>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_shared((const void*)k_three_center<LA, LB, LP>, smem);
+    if (e != cudaSuccess) return e;
     const int share = triple_share(ntasks, nalist, SH::SPW, 4, max_npp, SH::TPR, kShareTasks);
     const int per_cta = 4 * (SH::SPW / share);
     dim3 grid(ntasks, (nalist + per_cta - 1) / per_cta);  // 4 warps of SPW / share shells
@@ -772,8 +769,8 @@ cudaError_t launch_three_center(int la, int lb, const PairTask* tasks, int ntask
 
 template <int LA, int LB, int LP>
 static bool three_center_one_fits(int max_npp) {
-    return shared_fits(k_three_center<LA, LB, LP>,
-                       sizeof(double) * ((size_t)max_npp * PairLayout<LA, LB>::STRIDE + ThreeCenterShape<LA, LB, LP>::R_DOUBLES));
+    const size_t doubles = (size_t)max_npp * PairLayout<LA, LB>::STRIDE + ThreeCenterShape<LA, LB, LP>::R_DOUBLES;
+    return allow_shared((const void*)k_three_center<LA, LB, LP>, sizeof(double) * doubles) == cudaSuccess;
 }
 
 bool three_center_fits(int la, int lb, int max_npp, const int* count) {
@@ -781,7 +778,8 @@ bool three_center_fits(int la, int lb, int max_npp, const int* count) {
 #define HF_3CF(LA, LB, LP) (count[LP] == 0 || three_center_one_fits<LA, LB, LP>(max_npp))
 #define HF_3CF_P(LA, LB)                                                                                       \
     if (la == LA && lb == LB)                                                                                  \
-        fits = shared_fits(k_pair_data<LA, LB>, sizeof(double) * (size_t)max_npp * PairLayout<LA, LB>::STRIDE) && \
+        fits = allow_shared((const void*)k_pair_data<LA, LB>,                                                  \
+                            sizeof(double) * (size_t)max_npp * PairLayout<LA, LB>::STRIDE) == cudaSuccess &&   \
                HF_3CF(LA, LB, 0) && HF_3CF(LA, LB, 1) && HF_3CF(LA, LB, 2) && HF_3CF(LA, LB, 3) && HF_3CF(LA, LB, 4);
     HF_3CF_P(0, 0)
     HF_3CF_P(0, 1)

@@ -88,6 +88,14 @@ struct Branches {
     }
 };
 
+// Lets `kernel` be launched with smem bytes of dynamic shared memory, or says that it
+// cannot (cudaErrorInvalidValue). Up to kPlainShared that needs nothing (the static
+// tables count against the 48 KB default too); past it the kernel's limit is raised
+// once per device to all that its static part leaves. Set to each launch's own size, a
+// host thread with a smaller basis could lower it between another's setting and launch.
+constexpr size_t kPlainShared = 32 * 1024;
+cudaError_t allow_shared(const void* kernel, size_t smem);
+
 // The constant tables every integral kernel reads (each translation unit with
 // such kernels holds its own __constant__ copy): Cartesian-to-spherical
 // matrices, the (t, u, v) of each tetrahedral index up to order 8 and the

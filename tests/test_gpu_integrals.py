@@ -124,3 +124,29 @@ def test_shell_pairs_at_the_shared_memory_limit(n_prim, fits):
     ctx.upload(water_orb, aux)
     ctx.build()
     np.testing.assert_allclose(ctx.three_center(), dfrhf.three_center(aux, water_orb), atol=ORACLE_TOL, rtol=0)
+
+
+def test_bases_of_several_sizes_at_once():
+    """The kernels' shared memory limits are the process's: a thread with small pairs must not lower them
+    between another's setting and launch (a launch failed about once in 300 builds when each set its own)."""
+    import threading
+
+    mol = molecule("water")
+    aux = tables(mol)[1]
+    failures = []
+
+    def build(n_prim):
+        try:
+            for _ in range(150):
+                ctx = context_for(contracted(n_prim, mol.positions), aux)
+                ctx.build()
+                ctx.close()
+        except Exception as error:  # noqa: BLE001 - raised again on the main thread
+            failures.append(error)
+
+    threads = [threading.Thread(target=build, args=(n_prim,)) for n_prim in (5, 4, 3, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
