@@ -340,12 +340,14 @@ class Context:
         self.check(self.lib.hf_boys(self.handle, t.ctypes.data, t.shape[0], int(n_max), out.ctypes.data), "hf_boys")
         return out
 
-    def set_wait_limit(self, seconds: float, stall_next_build: bool = False) -> None:
+    def set_wait_limit(self, seconds: float, stall_next_build: bool = False, stall_next_coulomb: bool = False) -> None:
         """Limit of the split-BF16 exchange's device waits; ``stall_next_build``
         makes the next split-BF16 build wait once on a barrier that nothing
-        completes (it then returns HF_ERR_TIMEOUT, raised as BackendError)."""
-        self.check(self.lib.hf_set_wait_limit(self.handle, int(round(seconds * 1e9)), int(stall_next_build)),
-                   "hf_set_wait_limit")
+        completes (it then returns HF_ERR_TIMEOUT, raised as BackendError),
+        ``stall_next_coulomb`` the next J build for a packet that nothing sends
+        (with the same outcome)."""
+        stall = 2 if stall_next_coulomb else int(bool(stall_next_build))
+        self.check(self.lib.hf_set_wait_limit(self.handle, int(round(seconds * 1e9)), stall), "hf_set_wait_limit")
 
     def coulomb_static_device(self, d, out) -> None:
         """J into ``out`` through hf_coulomb_static, the build that allocates no

@@ -100,6 +100,7 @@ struct hf_ctx {
     // bounded device waits of the split-BF16 exchange (hf_set_wait_limit)
     uint64_t wait_ns = 2000000000ull;  // 2 s: far above any legitimate wait there
     int stall_next = 0;                // the next split-BF16 build runs the stall self-test
+    int stall_coulomb = 0;             // the next one-pass J build runs its own
 };
 
 namespace {
@@ -846,7 +847,8 @@ int hf_set_wait_limit(hf_ctx* ctx, int64_t wait_ns, int stall_next_build) {
     if (wait_ns < 1000 || wait_ns > 60000000000ll)
         return fail(ctx, HF_ERR_ARG, "the wait limit lies between 1 us and 60 s (got " + std::to_string(wait_ns) + " ns)");
     ctx->wait_ns = (uint64_t)wait_ns;
-    ctx->stall_next = stall_next_build ? 1 : 0;
+    ctx->stall_next = stall_next_build != 0 && stall_next_build != 2;
+    ctx->stall_coulomb = stall_next_build == 2;
     return HF_OK;
 }
 
@@ -1340,7 +1342,9 @@ static int coulomb_run(hf_ctx* ctx, const JkPlan& p, bool fused, const double* D
     }
     std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
     if (coulomb_fused_cooperative(p)) lock.lock();
-    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, ctx->wait_ns, ctx->stream));
+    const int stall = ctx->stall_coulomb;
+    ctx->stall_coulomb = 0;
+    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, ctx->wait_ns, stall, ctx->stream));
     ++ctx->stats.kernel_launches;
     if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     const int s = check_async(ctx, what);

@@ -76,6 +76,7 @@ struct FusedArgs {
     double2* jpart;             // [gq][ge * pp]
     unsigned long long* jflag;  // [gq][ge]
     uint32_t tag;               // tags of this launch: tag + row block, and tag + blocks for J
+    uint32_t sent;              // ... as the CTAs send them: `tag`, or, in the self-test, tags that none waits for
     uint32_t* stop;             // becomes `tag` when a wait has run out (device memory: polled by every wait)
     int* err;                   // ... and this becomes 1 (host memory: only ever written)
     uint64_t wait_ns;
@@ -144,16 +145,25 @@ __device__ __forceinline__ void give_up(const FusedArgs& a) {
     *(volatile int*)a.err = 1;
 }
 
-// Bounded wait for a barrier of this CTA: past the limit the error is recorded and the
-// caller goes on (its results are then undefined, its accesses stay in bounds).
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const FusedArgs& a) {
-    if (mbar_try(bar, parity)) return;
+// Bounded wait for a barrier of this CTA: past the limit, or once any wait of the launch has run
+// out, the caller goes on (its results are then undefined, its accesses stay in bounds). A collector
+// that has given up passes through all remaining row blocks at once, and its arrivals no longer fit
+// the workers' parities: a worker that waited for each of them ran out for each of them.
+// The clock and the stop word are read out of line, after the waits that matter: with the clock in
+// the loop (H2O)32 took 2.08 ms, with both 2.15, this way 1.83.
+__device__ __noinline__ void mbar_wait_long(uint64_t* bar, uint32_t parity, const FusedArgs& a) {
     const uint64_t start = now_ns();
     for (uint32_t i = 1; !mbar_try(bar, parity); ++i)
-        if ((i & 255) == 0 && now_ns() - start > 4 * a.wait_ns) {
-            give_up(a);
-            return;
+        if ((i & 15) == 0) {
+            const bool late = now_ns() - start > 4 * a.wait_ns;
+            if (late) give_up(a);
+            if (late || stopped(a)) return;
         }
+}
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const FusedArgs& a) {
+    for (int i = 0; i < 256; ++i)
+        if (mbar_try(bar, parity)) return;
+    mbar_wait_long(bar, parity, a);
 }
 
 // A warp's pieces of one row to and from tensor memory: W 32-bit registers per lane, W columns.
@@ -376,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
                     double v = 0.0;
                     for (int i = 0; i < a.tpq; i += 32) v += p[q * a.tpq + i];
                     if (a.ge == 1) c[q] = v;
-                    else put_packet(out + q * a.ge, v, a.tag + g);
+                    else put_packet(out + q * a.ge, v, a.sent + g);
                 }
             for (int q = 0; few && q < qb; ++q, p += a.tpq) {
                 double v = 0.0, w = 0.0;
@@ -390,7 +400,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
                 for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
                 if (lane == 0) {
                     if (a.ge == 1) c[q] = v;
-                    else put_packet(out + q * a.ge, v, a.tag + g);
+                    else put_packet(out + q * a.ge, v, a.sent + g);
                 }
             }
             __syncwarp();
@@ -603,12 +613,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
 #pragma unroll
         for (int k = 0; k < EPT; ++k)
             if (on >> k & 1) __stcg(a.jpart + ((int64_t)grp * a.ge + e) * a.pp + k * a.tpq + tl, acc[k]);
-    const uint32_t last = a.tag + a.blocks;
-    const unsigned long long done = ((unsigned long long)last << 32) | (uint32_t)~last;
+    auto flag = [&](uint32_t tag) { return ((unsigned long long)(tag + a.blocks) << 32) | (uint32_t)~(tag + a.blocks); };
+    const unsigned long long done = flag(a.tag);
     bar_sync(kBarW, kWorkers);
     if (tid == 0) {
         __threadfence();
-        *(volatile unsigned long long*)(a.jflag + grp * a.ge + e) = done;
+        *(volatile unsigned long long*)(a.jflag + grp * a.ge + e) = flag(a.sent);
     }
     if (tid < a.gq) {
         const volatile unsigned long long* f = a.jflag + tid * a.ge + e;
@@ -765,7 +775,7 @@ std::mutex& cooperative_mutex(int device) {
 }
 
 cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
-                                PacketSpace& held, int* err, uint64_t wait_ns, cudaStream_t stream) {
+                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, cudaStream_t stream) {
     const FusedShape f = plan_coulomb(p, device_sms());
     if (!f.ept) return cudaErrorInvalidValue;
     FusedArgs a = f.a;
@@ -783,7 +793,7 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     a.stop = reinterpret_cast<uint32_t*>(a.jflag + (size_t)a.gq * a.ge);
     a.jpart = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(a.packets) + tagged_bytes(a));
     // no word of the tagged part holds a tag of this build: it holds smaller tags of builds of this shape, or zeros
-    const uint32_t tags = (uint32_t)a.blocks + 1;
+    const uint32_t tags = ((uint32_t)a.blocks + 1) * (stall ? 2 : 1);
     if (held.next == 0 || held.n != p.n || held.naux != p.naux || held.next > UINT32_MAX - tags) {
         held.next = 0;
         const cudaError_t e = cudaMemsetAsync(a.packets, 0, tagged_bytes(a), stream);
@@ -791,6 +801,7 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
         held = PacketSpace{p.n, p.naux, 1};
     }
     a.tag = held.next;
+    a.sent = a.tag + tags - ((uint32_t)a.blocks + 1);
     held.next += tags;
     a.err = err;
     a.wait_ns = wait_ns;

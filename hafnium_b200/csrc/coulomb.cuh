@@ -26,12 +26,12 @@ struct PacketSpace {
 
 // J = scale * sum_q (B_q . D) B_q, J full n x n. The grid's CTAs wait on one another,
 // bounded by wait_ns; past it *err (device-visible, 0 before) becomes 1 and J is
-// undefined. A small grid is one thread-block cluster; a larger one is cooperative
+// undefined (stall: a self-test in which one CTA's first packets are not sent). A small grid is one thread-block cluster; a larger one is cooperative
 // (coulomb_fused_cooperative): hold cooperative_mutex(device) from its launch to its
 // completion, since two such grids in flight could each hold SMs that the other waits for.
 bool coulomb_fused_cooperative(const JkPlan& p);
 cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
-                                PacketSpace& held, int* err, uint64_t wait_ns, cudaStream_t stream);
+                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, cudaStream_t stream);
 
 std::mutex& cooperative_mutex(int device);
 

@@ -57,6 +57,32 @@ def test_coulomb_of_every_layout(n, n_aux):
     assert float(((inplace - expected).abs() / bound).max()) < 1.0
 
 
+# one cluster, groups that meet only in J, collectors by lanes, by warps and through owners, few and many
+# row blocks
+@pytest.mark.parametrize("n,n_aux", [(24, 113), (48, 226), (192, 64), (288, 150), (777, 70), (777, 450)])
+def test_a_wait_that_runs_out_ends_the_build(n, n_aux):
+    """A J build whose CTAs wait for packets that none sends gives up after its limit. The builds after it,
+    in the same workspace, are right again."""
+    import time
+
+    import torch
+
+    from hafnium_b200.errors import BackendError
+
+    two_body = hydrogens(n, n_aux)
+    d = torch.randn((n, n), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+    d = d + d.T
+    before = two_body.coulomb(d)
+    two_body.context.set_wait_limit(0.25, stall_next_coulomb=True)
+    start = time.perf_counter()
+    with pytest.raises(BackendError, match="a wait"):
+        two_body.coulomb(d)
+    # the limit once, not once for each row block
+    assert 0.2 < time.perf_counter() - start < 0.9
+    for _ in range(2):
+        assert torch.equal(two_body.coulomb(d), before)
+
+
 def test_the_first_coulomb_builds_of_a_process():
     """The packets between CTAs are told by their tags from what the memory held before: a fresh process,
     whose tags start anew in memory that the build's integer lists have just used."""
