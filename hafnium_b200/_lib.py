@@ -344,8 +344,8 @@ class Context:
         """Limit of the split-BF16 exchange's device waits; ``stall_next_build``
         makes the next split-BF16 build wait once on a barrier that nothing
         completes (it then returns HF_ERR_TIMEOUT, raised as BackendError),
-        ``stall_next_coulomb`` the next J build for a packet that nothing sends
-        (with the same outcome)."""
+        ``stall_next_coulomb`` the next J build for a packet that nothing sends (it
+        then takes its two-pass form and succeeds)."""
         stall = 2 if stall_next_coulomb else int(bool(stall_next_build))
         self.check(self.lib.hf_set_wait_limit(self.handle, int(round(seconds * 1e9)), stall), "hf_set_wait_limit")
 

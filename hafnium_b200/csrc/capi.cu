@@ -1322,37 +1322,52 @@ static JkPlan plan_of(const hf_ctx* ctx) {
     return p;
 }
 
-// The one-pass J build where it applies, else the two-pass one; returns once J is
-// complete. work holds coulomb_doubles(ctx, p).
-static size_t coulomb_doubles(const hf_ctx* ctx, const JkPlan& p, bool* fused) {
-    const size_t need = ctx->h_flag ? coulomb_fused_work_doubles(p) : 0;
-    *fused = need > 0;
-    return need ? need : (size_t)coulomb_work_doubles(p);
+// Limit of the one-pass J build's waits between its CTAs, which take microseconds. It is
+// not hf_set_wait_limit's: a caller who sets a short one for the split-BF16 pipeline
+// would have every J built twice.
+constexpr uint64_t kCoulombWaitNs = 250000000ull;
+
+// How a J build runs: the one-pass form where it applies, else the two-pass one. When a
+// wait of the one-pass build runs out, J is built after it in two passes, which wait for
+// nothing; that needs D as it was, so a D that J overlaps is copied first.
+struct CoulombRun {
+    bool fused, copy;
+    size_t builds, doubles;  // scratch of either form; with the copy of D behind it
+};
+
+static CoulombRun coulomb_plan(const hf_ctx* ctx, const JkPlan& p, const double* D, const double* J) {
+    const size_t nn = (size_t)p.n * p.n, plain = (size_t)coulomb_work_doubles(p);
+    const size_t one = ctx->h_flag ? coulomb_fused_work_doubles(p) : 0;
+    CoulombRun r{one > 0, one > 0 && D < J + nn && J < D + nn, std::max(one, plain), 0};
+    r.doubles = r.builds + (r.copy ? nn : 0);
+    return r;
 }
 
-static int coulomb_run(hf_ctx* ctx, const JkPlan& p, bool fused, const double* D, double* J, double* work,
+// Returns once J is complete. work holds run.doubles.
+static int coulomb_run(hf_ctx* ctx, const JkPlan& p, const CoulombRun& run, const double* D, double* J, double* work,
                        PacketSpace& held, double* host_out, const char* what) {
     const size_t bytes = sizeof(double) * (size_t)p.n * p.n;
-    if (!fused) {
-        held.next = 0;
-        HF_CU(coulomb_build(p, D, J, work, ctx->stream));
-        ctx->stats.kernel_launches += 4;
+    if (run.copy) {
+        HF_CU(cudaMemcpyAsync(work + run.builds, D, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        D = work + run.builds;
+    }
+    if (run.fused) {
+        std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
+        if (coulomb_fused_cooperative(p)) lock.lock();
+        const int stall = ctx->stall_coulomb;
+        ctx->stall_coulomb = 0;
+        HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, kCoulombWaitNs, stall, ctx->stream));
+        ++ctx->stats.kernel_launches;
         if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        return check_async(ctx, what);
-    }
-    std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
-    if (coulomb_fused_cooperative(p)) lock.lock();
-    const int stall = ctx->stall_coulomb;
-    ctx->stall_coulomb = 0;
-    HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, ctx->wait_ns, stall, ctx->stream));
-    ++ctx->stats.kernel_launches;
-    if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    const int s = check_async(ctx, what);
-    if (s == HF_OK && *(volatile int*)ctx->h_flag != 0) {
+        const int s = check_async(ctx, what);
+        if (s != HF_OK || *(volatile int*)ctx->h_flag == 0) return s;
         *(volatile int*)ctx->h_flag = 0;
-        return fail(ctx, HF_ERR_TIMEOUT, std::string(what) + ": a wait between the kernel's CTAs ran out");
     }
-    return s;
+    held.next = 0;
+    HF_CU(coulomb_build(p, D, J, work, ctx->stream));
+    ctx->stats.kernel_launches += 4;
+    if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    return check_async(ctx, what);
 }
 
 int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
@@ -1362,19 +1377,18 @@ int hf_coulomb(hf_ctx* ctx, const double* D, double* J, int on_device) {
     const JkPlan p = plan_of(ctx);
     const size_t nn = (size_t)ctx->n * ctx->n;
     int s;
-    bool fused = false;
-    const size_t need = coulomb_doubles(ctx, p, &fused);
-    if ((s = ensure_work(ctx, sizeof(double) * need)) != HF_OK) return s;
     const double* dD = D;
     double* dJ = J;
     if (!on_device) {
-        if ((s = ensure_io(ctx, 2 * nn * sizeof(double))) != HF_OK) return s;
+        if ((s = ensure_io(ctx, 2 * nn * 8)) != HF_OK) return s;
         HF_CU(cudaMemcpyAsync(ctx->d_io, D, nn * 8, cudaMemcpyHostToDevice, ctx->stream));
         dD = ctx->d_io;
         dJ = ctx->d_io + nn;
     }
+    const CoulombRun run = coulomb_plan(ctx, p, dD, dJ);
+    if ((s = ensure_work(ctx, sizeof(double) * run.doubles)) != HF_OK) return s;
     time_begin(ctx);
-    s = coulomb_run(ctx, p, fused, dD, dJ, ctx->d_work, ctx->packets, on_device ? nullptr : J, "hf_coulomb");
+    s = coulomb_run(ctx, p, run, dD, dJ, ctx->d_work, ctx->packets, on_device ? nullptr : J, "hf_coulomb");
     ctx->stats.ms_coulomb = time_end(ctx);
     return s;
 }
@@ -2349,9 +2363,10 @@ int hf_boys(hf_ctx* ctx, const double* t, int64_t count, int n_max, double* out)
 // already fully reserved by its own pool allocator (a cudaMalloc would fail or
 // fragment that pool), or a latency-critical loop in which a cudaMalloc /
 // cudaFree pair, which can synchronise the device, is not allowed. For them
-// hf_coulomb_static runs the same J build as hf_coulomb but takes its scratch
-// (the weighted packed density, the fitting charges and the packed J) from the
-// file-scope array below instead of from an allocation. The caller still passes
+// hf_coulomb_static runs the same J build as hf_coulomb but takes its scratch (the
+// weighted packed density, the fitting charges and the packed J of the two-pass form,
+// which is the larger; the packets and partial sums of the one-pass form; a density that
+// J overwrites) from the file-scope array below instead of from an allocation. The caller still passes
 // the density and J as device pointers.
 //
 // Limits: n_ao <= kStaticMaxAo (1536, 24 tiles of 64) and n_aux <= kStaticMaxAux
@@ -2406,9 +2421,12 @@ extern "C" int hf_coulomb_static(hf_ctx* ctx, const double* density, double* cou
     int s = static_scratch(ctx, &scratch);
     if (s != HF_OK) return s;
     const JkPlan p = plan_of(ctx);
-    bool fused = false;
-    if (coulomb_doubles(ctx, p, &fused) > (size_t)kStaticScratchDoubles)
-        return fail(ctx, HF_ERR_ARG, "scratch size exceeded");
-    return coulomb_run(ctx, p, fused, density, coulomb, scratch, g_scratch_packets[ctx->device], nullptr,
+    CoulombRun run = coulomb_plan(ctx, p, density, coulomb);
+    if (run.doubles > (size_t)kStaticScratchDoubles) {  // no room for the copy of D: two passes need none
+        const size_t plain = (size_t)coulomb_work_doubles(p);
+        run = CoulombRun{false, false, plain, plain};
+    }
+    if (run.doubles > (size_t)kStaticScratchDoubles) return fail(ctx, HF_ERR_ARG, "scratch size exceeded");
+    return coulomb_run(ctx, p, run, density, coulomb, scratch, g_scratch_packets[ctx->device], nullptr,
                        "hf_coulomb_static");
 }

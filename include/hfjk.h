@@ -121,8 +121,9 @@ int hf_release_retained(int device);
  * stall_next_build set, the next split-BF16 build waits once on a barrier that
  * nothing completes, so that path can be tested without a fault. With
  * stall_next_build = 2 it is the next J build whose thread blocks wait once for
- * a packet that none sends (the limit holds for that build's waits too). No
- * reference counterpart (the reference has no device code). */
+ * a packet that none sends: hf_coulomb's own waits have a fixed limit of 0.25 s,
+ * and past it J is built in the two-pass form, which waits for nothing, so the
+ * call succeeds. No reference counterpart (the reference has no device code). */
 int hf_set_wait_limit(hf_ctx* ctx, int64_t wait_ns, int stall_next_build);
 
 /* Upload the orbital and auxiliary shells (replaces the _kernels.ShellTable

@@ -57,30 +57,47 @@ def test_coulomb_of_every_layout(n, n_aux):
     assert float(((inplace - expected).abs() / bound).max()) < 1.0
 
 
-# one cluster, groups that meet only in J, collectors by lanes, by warps and through owners, few and many
-# row blocks
+# one cluster, groups that meet only in J, collectors by lanes, by warps and through owners, few and
+# many row blocks
 @pytest.mark.parametrize("n,n_aux", [(24, 113), (48, 226), (192, 64), (288, 150), (777, 70), (777, 450)])
-def test_a_wait_that_runs_out_ends_the_build(n, n_aux):
-    """A J build whose CTAs wait for packets that none sends gives up after its limit. The builds after it,
-    in the same workspace, are right again."""
+def test_a_wait_that_runs_out_costs_time_only(n, n_aux):
+    """A J build whose CTAs wait for packets that none sends gives up after its limit, and J is built in two
+    passes, also a J that overwrites D. The builds after it, in the same workspace, are one-pass again."""
     import time
 
     import torch
-
-    from hafnium_b200.errors import BackendError
 
     two_body = hydrogens(n, n_aux)
     d = torch.randn((n, n), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
     d = d + d.T
     before = two_body.coulomb(d)
-    two_body.context.set_wait_limit(0.25, stall_next_coulomb=True)
+    torch.cuda.synchronize()
+    launches = two_body.context.stats()["kernel_launches"]
+    two_body.context.set_wait_limit(1e-6)  # the split-BF16 pipeline's
+    assert torch.equal(two_body.coulomb(d), before)
+    assert two_body.context.stats()["kernel_launches"] == launches + 1
+    two_body.context.set_wait_limit(2.0, stall_next_coulomb=True)
     start = time.perf_counter()
-    with pytest.raises(BackendError, match="a wait"):
-        two_body.coulomb(d)
-    # the limit once, not once for each row block
+    late = two_body.coulomb(d)
+    torch.cuda.synchronize()
+    # the limit of 0.25 s once, not once for each row block
     assert 0.2 < time.perf_counter() - start < 0.9
+    assert two_body.context.stats()["kernel_launches"] > launches + 2
+    # both sum n^2 and n_aux rounded products, in two orders (the bound of the first test, for each)
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = two_body.orbital_tensor(eye, eye).abs()
+    size = torch.einsum("quv,q->uv", b, torch.einsum("quv,uv->q", b, d.abs()))
+    assert bool(((late - before).abs() <= 2 * 2.3e-16 * (n * n + n_aux) * size).all())
+    assert torch.equal(two_body.coulomb(d), before)
+    inplace = d.clone()
+    two_body.context.set_wait_limit(2.0, stall_next_coulomb=True)
+    two_body.context.coulomb_device(inplace, inplace)
+    assert bool(((inplace - before).abs() <= 2 * 2.3e-16 * (n * n + n_aux) * size).all())
     for _ in range(2):
         assert torch.equal(two_body.coulomb(d), before)
+    inplace = d.clone()
+    two_body.context.coulomb_device(inplace, inplace)
+    assert torch.equal(inplace, before)
 
 
 def test_the_first_coulomb_builds_of_a_process():
