@@ -62,6 +62,10 @@ constexpr int kTmemDoubles = 64;         // a worker thread's share of tensor me
 constexpr int kParts = 2;                 // shared buffers of partial sums
 constexpr int kCluster = 8;               // grids up to this size are one thread-block cluster
 constexpr int kFewRows = 8;               // blocks of more rows are summed over a warp by the workers
+// Rows of one running sum of J; longer ones are added up in memory. One sum over all rows of a group
+// erred by 2.1e-15 of J at (H2O)32, five times as much as the two-pass form's slabs (4.1e-16); sums of
+// 128 rows err by 4.6e-16, of 64 by 3.7e-16. Writing them out is 0.16 of 1.97 ms there.
+constexpr int kChain = 64;
 constexpr int kBarW = 1, kBarEnd = 2;    // named barriers: workers; workers and publisher at the end
 
 struct FusedArgs {
@@ -90,6 +94,8 @@ struct FusedArgs {
     int ns;       // packet slots
     int rows;     // rows per group
     int blocks;   // row blocks per group
+    int flush;    // row blocks between two additions of the sums of J to jsum
+    double2* jsum;  // [gq * ge][ql][pp]
 };
 
 __device__ __forceinline__ void bar_sync(int id, int threads) {
@@ -480,6 +486,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
     double2 acc[EPT];
 #pragma unroll
     for (int k = 0; k < EPT; ++k) acc[k] = make_double2(0.0, 0.0);
+    // this thread's own entries of jsum: nobody else touches them
+    auto sums_at = [&] { return a.jsum + ((int64_t)blockIdx.x * a.ql + lq) * a.pp + tl; };
+    auto add_up = [&](bool more) {
+        double2* t = sums_at();
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) {
+            if (on >> k & 1) {
+                const double2 v = more ? __ldcg(t + k * a.tpq) : make_double2(0.0, 0.0);
+                __stcg(t + k * a.tpq, make_double2(v.x + acc[k].x, v.y + acc[k].y));
+            }
+            acc[k] = make_double2(0.0, 0.0);
+        }
+    };
+    auto take_sums = [&] {
+        const double2* t = sums_at();
+#pragma unroll
+        for (int k = 0; k < EPT; ++k)
+            if (on >> k & 1) {
+                const double2 v = __ldcg(t + k * a.tpq);
+                acc[k].x += v.x;
+                acc[k].y += v.y;
+            }
+    };
     if (mine) {
         // weights: D[mu][nu] + D[nu][mu] above the diagonal, D[mu][mu] on it, 0 below and past n
         double2 d[EPT];
@@ -497,6 +526,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
         const uint32_t mine_tmem = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * (2 * kTmemDoubles);
         int slot = 0, buf = 0, bpar = 1, put = 0;  // g modulo the smem ring, kParts and lag
         int get = 0, hbuf = 0, hpar = 0;  // the same for the block to be used
+        int left = a.flush;
         for (int g = 0; g < a.blocks + a.lag - 1; ++g) {
             if (g < a.blocks) {
                 issue(g + kPrefetch);
@@ -566,9 +596,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
                     hpar ^= 1;
                 }
                 get = get == a.lag - 1 ? 0 : get + 1;
+                if (--left == 0) {
+                    left = a.flush;
+                    add_up(h >= a.flush);
+                }
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        if (a.blocks >= a.flush) take_sums();
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     bar_arrive(kBarEnd, kWorkers + 32);
@@ -635,14 +670,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
     const int share = (a.pp + a.gq - 1) / a.gq;
     for (int i = grp * share + tid; i < min(a.pp, (grp + 1) * share); i += kWorkers) {
         if (e * a.pp + i >= a.total) break;
-        double2 v = make_double2(0.0, 0.0);
-#pragma unroll 8
-        for (int r = 0; r < a.gq; ++r) {
-            const double2 x = __ldcg(a.jpart + ((int64_t)r * a.ge + e) * a.pp + i);
-            v.x += x.x;
-            v.y += x.y;
-        }
-        store(e * a.pp + i, v);
+        double2 v[4] = {};
+#pragma unroll 2
+        for (int r = 0; r < a.gq; r += 4)
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (r + m < a.gq) {
+                    const double2 x = __ldcg(a.jpart + ((int64_t)(r + m) * a.ge + e) * a.pp + i);
+                    v[m].x += x.x;
+                    v[m].y += x.y;
+                }
+        store(e * a.pp + i, make_double2((v[0].x + v[1].x) + (v[2].x + v[3].x), (v[0].y + v[1].y) + (v[2].y + v[3].y)));
     }
 }
 
@@ -729,6 +767,7 @@ FusedShape plan_coulomb(const JkPlan& p, int sms) {
     const int qb = a.ql * a.b;
     a.blocks = (a.rows + qb - 1) / qb;
     a.lag = std::min(a.lag, a.blocks);
+    a.flush = std::max(1, kChain / a.b);
     a.nr = a.lag + 2;
     a.ns = 2 * a.lag + 2;
     f.smem = 8 * (size_t)(2 * kParts + a.nr) + 8 * ((size_t)kParts * qb * a.tpq + a.nr * qb) + 32 +
@@ -739,6 +778,7 @@ FusedShape plan_coulomb(const JkPlan& p, int sms) {
 size_t packet_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b * a.ge; }
 size_t sum_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b; }
 size_t jpart_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ge * a.pp; }
+size_t jsum_bytes(const FusedArgs& a) { return a.blocks >= a.flush ? (size_t)16 * a.gq * a.ge * a.ql * a.pp : 0; }
 
 size_t flag_bytes(const FusedArgs& a) { return ((size_t)8 * a.gq * a.ge + 15) / 16 * 16 + 16; }  // and the stop word
 // what a build tells from older contents by its tags, at the front of the workspace
@@ -761,7 +801,7 @@ int device_sms() {
 size_t coulomb_fused_work_doubles(const JkPlan& p) {
     const FusedShape f = plan_coulomb(p, device_sms());
     if (!f.ept) return 0;
-    return (tagged_bytes(f.a) + jpart_bytes(f.a)) / 8 + 2;
+    return (tagged_bytes(f.a) + jpart_bytes(f.a) + jsum_bytes(f.a)) / 8 + 2;
 }
 
 bool coulomb_fused_cooperative(const JkPlan& p) {
@@ -792,6 +832,7 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     a.jflag = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(a.sums) + sum_bytes(a));
     a.stop = reinterpret_cast<uint32_t*>(a.jflag + (size_t)a.gq * a.ge);
     a.jpart = reinterpret_cast<double2*>(reinterpret_cast<uint8_t*>(a.packets) + tagged_bytes(a));
+    a.jsum = a.jpart + (size_t)a.gq * a.ge * a.pp;
     // no word of the tagged part holds a tag of this build: it holds smaller tags of builds of this shape, or zeros
     const uint32_t tags = ((uint32_t)a.blocks + 1) * (stall ? 2 : 1);
     if (held.next == 0 || held.n != p.n || held.naux != p.naux || held.next > UINT32_MAX - tags) {

@@ -57,6 +57,42 @@ def test_coulomb_of_every_layout(n, n_aux):
     assert float(((inplace - expected).abs() / bound).max()) < 1.0
 
 
+def pairwise(x):
+    """The sum over the first axis, halved again and again: its error is that of log2 of the terms' count."""
+    import torch
+
+    while x.shape[0] > 1:
+        if x.shape[0] & 1:
+            x = torch.cat([x, torch.zeros_like(x[:1])])
+        x = x[0::2] + x[1::2]
+    return x[0]
+
+
+@pytest.mark.parametrize("n,n_aux", [(450, 1200), (800, 2000)])
+def test_the_running_sums_of_j_are_short(n, n_aux):
+    """Rounding errors of a running sum add up like its partial sums' squares; J errs no more than sums of 64
+    rows, added up, do (one sum over all rows errs five times as much)."""
+    import torch
+
+    two_body = hydrogens(n, n_aux)
+    c = torch.randn((n, 40), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+    d = c @ c.T
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = two_body.orbital_tensor(eye, eye)
+    charges = torch.stack([pairwise((row * d).reshape(-1)) for row in b])
+    sums, squares = [], torch.zeros_like(d)
+    for q in range(0, n_aux, 64):
+        terms = b[q:q + 64] * charges[q:q + 64, None, None]
+        sums.append(pairwise(terms))
+        squares += (terms.cumsum(0) ** 2).sum(0)
+    totals = torch.stack(sums)
+    squares += (totals.cumsum(0) ** 2).sum(0)
+    # each rounding errs by at most 2^-53 of the partial sum, 1 / sqrt(3) of that in the mean square; twice
+    # that for the charges' own errors, which are of the size of one more addition
+    expected = 2 * 2.0**-53 / 3**0.5 * float(squares.sum().sqrt())
+    assert float((two_body.coulomb(d) - pairwise(totals)).norm()) < expected
+
+
 # one cluster, groups that meet only in J, collectors by lanes, by warps and through owners, few and
 # many row blocks
 @pytest.mark.parametrize("n,n_aux", [(24, 113), (48, 226), (192, 64), (288, 150), (777, 70), (777, 450)])
