@@ -306,7 +306,9 @@ __host__ __device__ constexpr int tmem_width() {
     return EPT == 1 ? 4 : EPT == 2 ? 8 : 16;
 }
 
-template <int EPT>
+// LONG: a thread's rows are more than one running sum takes (without that code the small sizes, whose
+// registers it needs, are 3 % faster).
+template <int EPT, bool LONG>
 __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_constant__ FusedArgs a) {
     constexpr int TW = tmem_width<EPT>();
     extern __shared__ __align__(16) uint8_t smem[];
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
         const uint32_t mine_tmem = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * (2 * kTmemDoubles);
         int slot = 0, buf = 0, bpar = 1, put = 0;  // g modulo the smem ring, kParts and lag
         int get = 0, hbuf = 0, hpar = 0;  // the same for the block to be used
-        int left = a.flush;
+        [[maybe_unused]] int left = a.flush;
         for (int g = 0; g < a.blocks + a.lag - 1; ++g) {
             if (g < a.blocks) {
                 issue(g + kPrefetch);
@@ -596,14 +598,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
                     hpar ^= 1;
                 }
                 get = get == a.lag - 1 ? 0 : get + 1;
-                if (--left == 0) {
-                    left = a.flush;
-                    add_up(h >= a.flush);
-                }
+                if constexpr (LONG)
+                    if (--left == 0) {
+                        left = a.flush;
+                        add_up(h >= a.flush);
+                    }
             }
         }
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        if (a.blocks >= a.flush) take_sums();
+        if constexpr (LONG) take_sums();
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     bar_arrive(kBarEnd, kWorkers + 32);
@@ -670,23 +673,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
     const int share = (a.pp + a.gq - 1) / a.gq;
     for (int i = grp * share + tid; i < min(a.pp, (grp + 1) * share); i += kWorkers) {
         if (e * a.pp + i >= a.total) break;
-        double2 v[4] = {};
-#pragma unroll 2
-        for (int r = 0; r < a.gq; r += 4)
+        double2 v[4] = {};  // four chains: the sum errs half as much, and its loads are ahead of it
+        auto add = [&](int m, int r) {
+            const double2 x = __ldcg(a.jpart + ((int64_t)r * a.ge + e) * a.pp + i);
+            v[m].x += x.x;
+            v[m].y += x.y;
+        };
+        int r = 0;
+#pragma unroll 4
+        for (; r + 3 < a.gq; r += 4)
 #pragma unroll
-            for (int m = 0; m < 4; ++m)
-                if (r + m < a.gq) {
-                    const double2 x = __ldcg(a.jpart + ((int64_t)(r + m) * a.ge + e) * a.pp + i);
-                    v[m].x += x.x;
-                    v[m].y += x.y;
-                }
+            for (int m = 0; m < 4; ++m) add(m, r + m);
+        for (; r < a.gq; ++r) add(0, r);
         store(e * a.pp + i, make_double2((v[0].x + v[1].x) + (v[2].x + v[3].x), (v[0].y + v[1].y) + (v[2].y + v[3].y)));
     }
 }
 
-template <int EPT>
+template <int EPT, bool LONG>
 cudaError_t launch_fused(const FusedArgs& a, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(k_coulomb_fused<EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(k_coulomb_fused<EPT, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     // the grid's CTAs wait on one another: a cluster, or a cooperative grid
     cudaLaunchConfig_t c{};
@@ -705,8 +710,11 @@ cudaError_t launch_fused(const FusedArgs& a, size_t smem, cudaStream_t stream) {
     }
     c.attrs = at;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k_coulomb_fused<EPT>, a);
+    return cudaLaunchKernelEx(&c, k_coulomb_fused<EPT, LONG>, a);
 }
+
+// A thread's rows are more than one running sum takes.
+bool long_sums(const FusedArgs& a) { return a.blocks >= a.flush; }
 
 int64_t upper_pieces(int64_t n, int nt) {
     int64_t total = 0;
@@ -778,7 +786,7 @@ FusedShape plan_coulomb(const JkPlan& p, int sms) {
 size_t packet_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b * a.ge; }
 size_t sum_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ns * a.ql * a.b; }
 size_t jpart_bytes(const FusedArgs& a) { return (size_t)16 * a.gq * a.ge * a.pp; }
-size_t jsum_bytes(const FusedArgs& a) { return a.blocks >= a.flush ? (size_t)16 * a.gq * a.ge * a.ql * a.pp : 0; }
+size_t jsum_bytes(const FusedArgs& a) { return long_sums(a) ? (size_t)16 * a.gq * a.ge * a.ql * a.pp : 0; }
 
 size_t flag_bytes(const FusedArgs& a) { return ((size_t)8 * a.gq * a.ge + 15) / 16 * 16 + 16; }  // and the stop word
 // what a build tells from older contents by its tags, at the front of the workspace
@@ -846,11 +854,12 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     held.next += tags;
     a.err = err;
     a.wait_ns = wait_ns;
+    const bool more = long_sums(a);
     switch (f.ept) {
-        case 1: return launch_fused<1>(a, f.smem, stream);
-        case 2: return launch_fused<2>(a, f.smem, stream);
-        case 3: return launch_fused<3>(a, f.smem, stream);
-        case 4: return launch_fused<4>(a, f.smem, stream);
+        case 1: return more ? launch_fused<1, true>(a, f.smem, stream) : launch_fused<1, false>(a, f.smem, stream);
+        case 2: return more ? launch_fused<2, true>(a, f.smem, stream) : launch_fused<2, false>(a, f.smem, stream);
+        case 3: return more ? launch_fused<3, true>(a, f.smem, stream) : launch_fused<3, false>(a, f.smem, stream);
+        case 4: return more ? launch_fused<4, true>(a, f.smem, stream) : launch_fused<4, false>(a, f.smem, stream);
         default: return cudaErrorInvalidValue;
     }
 }
