@@ -63,9 +63,11 @@ constexpr int kParts = 2;                 // shared buffers of partial sums
 constexpr int kCluster = 8;               // grids up to this size are one thread-block cluster
 constexpr int kFewRows = 8;               // blocks of more rows are summed over a warp by the workers
 // Rows of one running sum of J; longer ones are added up in memory. One sum over all rows of a group
-// erred by 2.1e-15 of J at (H2O)32, five times as much as the two-pass form's slabs (4.1e-16); sums of
-// 128 rows err by 4.6e-16, of 64 by 3.7e-16. Writing them out is 0.16 of 1.97 ms there.
-constexpr int kChain = 64;
+// erred by 6.7e-16 of J at (H2O)16 and 2.1e-15 at (H2O)32, the two-pass form's slabs by 3.7e-16 and
+// 4.1e-16; sums of 128 rows err by 4.6e-16 at both, of 88 by 3.7e-16 and 3.8e-16 (of 64 by 3.1e-16 and
+// 3.7e-16). One addition of all CTAs' sums takes about 6 us, all CTAs at once: at different times each
+// held up the others ((H2O)32 1.93 -> 2.40 ms).
+constexpr int kChain = 88;
 constexpr int kBarW = 1, kBarEnd = 2;    // named barriers: workers; workers and publisher at the end
 
 struct FusedArgs {
@@ -306,8 +308,8 @@ __host__ __device__ constexpr int tmem_width() {
     return EPT == 1 ? 4 : EPT == 2 ? 8 : 16;
 }
 
-// LONG: a thread's rows are more than one running sum takes (without that code the small sizes, whose
-// registers it needs, are 3 % faster).
+// LONG: a thread's rows are more than one running sum takes. Without that code, whose registers they
+// need, the small sizes are 3 % faster.
 template <int EPT, bool LONG>
 __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_constant__ FusedArgs a) {
     constexpr int TW = tmem_width<EPT>();
@@ -343,20 +345,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
 
     const int lq = tid / a.tpq, tl = tid - lq * a.tpq;
     const bool mine = lq < a.ql;  // the same for a whole warp
-    int off[EPT];
+    // where the thread's pieces lie in a row: in registers, or, where the long sums need those, in shared memory
+    int4* kept = reinterpret_cast<int4*>(slots + (kPrefetch + 1) * a.b * EPT * lanes) + tid;
+    int off[4] = {0, 0, 0, 0};
     uint32_t on = 0;
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
         const int i = k * a.tpq + tl, idx = e * a.pp + i;
-        off[k] = 0;
         if (warp < kWorkers / 32 && mine && i < a.pp && idx < a.total) {
             int u, v;
             locate(idx, a.n, a.nt, off[k], u, v);
             on |= 1u << k;
         }
     }
+    if (LONG && warp < kWorkers / 32 && mine) *kept = make_int4(off[0], off[1], off[2], off[3]);
     auto issue = [&](int g) {
         if (g < a.blocks) {
+            if constexpr (LONG) {
+                const int4 o = *kept;
+                off[0] = o.x;
+                off[1] = o.y;
+                off[2] = o.z;
+                off[3] = o.w;
+            }
             for (int s = 0; s < a.b; ++s) {
                 const int q = q0 + g * qb + s * a.ql + lq;
                 if (q >= q1) break;
@@ -495,8 +506,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
             if (on >> k & 1) {
-                const double2 v = more ? __ldcg(t + k * a.tpq) : make_double2(0.0, 0.0);
-                __stcg(t + k * a.tpq, make_double2(v.x + acc[k].x, v.y + acc[k].y));
+                if (more) {  // additions that nothing waits for
+                    atomicAdd(&t[k * a.tpq].x, acc[k].x);
+                    atomicAdd(&t[k * a.tpq].y, acc[k].y);
+                } else {
+                    __stcg(t + k * a.tpq, acc[k]);
+                }
             }
             acc[k] = make_double2(0.0, 0.0);
         }
@@ -713,8 +728,6 @@ cudaError_t launch_fused(const FusedArgs& a, size_t smem, cudaStream_t stream) {
     return cudaLaunchKernelEx(&c, k_coulomb_fused<EPT, LONG>, a);
 }
 
-// A thread's rows are more than one running sum takes.
-bool long_sums(const FusedArgs& a) { return a.blocks >= a.flush; }
 
 int64_t upper_pieces(int64_t n, int nt) {
     int64_t total = 0;
@@ -726,6 +739,9 @@ int64_t upper_pieces(int64_t n, int nt) {
     }
     return total;
 }
+
+// A thread's rows are more than one running sum takes.
+bool long_sums(const FusedArgs& a) { return a.blocks >= a.flush; }
 
 constexpr int kMaxPieces = 4;         // pieces of a row per thread
 constexpr int64_t kSmallPieces = 20000;  // up to here one cluster of 8 CTAs holds everything (one water: 23.5 us, 27 spread out)
@@ -779,7 +795,7 @@ FusedShape plan_coulomb(const JkPlan& p, int sms) {
     a.nr = a.lag + 2;
     a.ns = 2 * a.lag + 2;
     f.smem = 8 * (size_t)(2 * kParts + a.nr) + 8 * ((size_t)kParts * qb * a.tpq + a.nr * qb) + 32 +
-             slot * (kPrefetch + 1) * a.b;
+             slot * (kPrefetch + 1) * a.b + (long_sums(a) ? (size_t)16 * a.ql * a.tpq : 0);
     return f;
 }
 

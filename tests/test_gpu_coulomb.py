@@ -70,7 +70,7 @@ def pairwise(x):
 
 @pytest.mark.parametrize("n,n_aux", [(450, 1200), (800, 2000)])
 def test_the_running_sums_of_j_are_short(n, n_aux):
-    """Rounding errors of a running sum add up like its partial sums' squares; J errs no more than sums of 64
+    """Rounding errors of a running sum add up like its partial sums' squares; J errs no more than sums of 88
     rows, added up, do (one sum over all rows errs five times as much)."""
     import torch
 
@@ -81,8 +81,8 @@ def test_the_running_sums_of_j_are_short(n, n_aux):
     b = two_body.orbital_tensor(eye, eye)
     charges = torch.stack([pairwise((row * d).reshape(-1)) for row in b])
     sums, squares = [], torch.zeros_like(d)
-    for q in range(0, n_aux, 64):
-        terms = b[q:q + 64] * charges[q:q + 64, None, None]
+    for q in range(0, n_aux, 88):
+        terms = b[q:q + 88] * charges[q:q + 88, None, None]
         sums.append(pairwise(terms))
         squares += (terms.cumsum(0) ** 2).sum(0)
     totals = torch.stack(sums)
