@@ -1352,11 +1352,15 @@ static int coulomb_run(hf_ctx* ctx, const JkPlan& p, const CoulombRun& run, cons
         D = work + run.builds;
     }
     if (run.fused) {
-        std::unique_lock<std::mutex> lock(cooperative_mutex(ctx->device), std::defer_lock);
-        if (coulomb_fused_cooperative(p)) lock.lock();
+        // what a caller has queued on a stream of its own may wait for another context's build: it must not
+        // stand between this build's turn and its grid, nor may what is queued behind the grid
+        const bool own = ctx->stream == ctx->own;
+        if (!own) HF_CU(cudaStreamSynchronize(ctx->stream));
+        CooperativeTurn turn(ctx->device);
         const int stall = ctx->stall_coulomb;
         ctx->stall_coulomb = 0;
-        HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, kCoulombWaitNs, stall, ctx->stream));
+        HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, kCoulombWaitNs, stall, turn,
+                                  own ? nullptr : ctx->ev1, ctx->stream));
         ++ctx->stats.kernel_launches;
         if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         const int s = check_async(ctx, what);

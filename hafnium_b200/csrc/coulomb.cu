@@ -46,6 +46,7 @@
 #include <mutex>
 
 #include "coulomb.cuh"
+#include "integrals.cuh"
 
 
 namespace hf {
@@ -706,7 +707,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_coulomb_fused(const __grid_cons
 
 template <int EPT, bool LONG>
 cudaError_t launch_fused(const FusedArgs& a, size_t smem, cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(k_coulomb_fused<EPT, LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = allow_shared((const void*)k_coulomb_fused<EPT, LONG>, smem);
     if (e != cudaSuccess) return e;
     // the grid's CTAs wait on one another: a cluster, or a cooperative grid
     cudaLaunchConfig_t c{};
@@ -828,18 +829,51 @@ size_t coulomb_fused_work_doubles(const JkPlan& p) {
     return (tagged_bytes(f.a) + jpart_bytes(f.a) + jsum_bytes(f.a)) / 8 + 2;
 }
 
-bool coulomb_fused_cooperative(const JkPlan& p) {
-    const FusedShape f = plan_coulomb(p, device_sms());
-    return f.ept && f.a.ge * f.a.gq > kCluster;
+namespace {
+struct Turns {
+    std::mutex mutex;
+    uint64_t last = 0;       // number of the last turn
+    bool busy = false;       // ... which has not been left
+    cudaStream_t stream{};   // ... its stream
+    cudaEvent_t mark{};      // ... and its event, if it has one
+    cudaEvent_t event{};     // for those that have none
+};
+Turns g_turns[64];
+Turns& turns_of(int device) { return g_turns[device >= 0 && device < 64 ? device : 0]; }
+}  // namespace
+
+std::mutex& CooperativeTurn::mutex() { return turns_of(device_).mutex; }
+
+cudaError_t CooperativeTurn::follow(cudaStream_t stream) {
+    Turns& t = turns_of(device_);
+    if (!t.busy) return cudaSuccess;
+    if (t.mark) return cudaStreamWaitEvent(stream, t.mark, 0);
+    cudaError_t e = t.event ? cudaSuccess : cudaEventCreateWithFlags(&t.event, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(t.event, t.stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, t.event, 0);
+    return e;
 }
 
-std::mutex& cooperative_mutex(int device) {
-    static std::mutex mutexes[64];
-    return mutexes[device >= 0 && device < 64 ? device : 0];
+cudaError_t CooperativeTurn::take(cudaStream_t stream, cudaEvent_t mark) {
+    Turns& t = turns_of(device_);
+    number_ = ++t.last;
+    t.busy = true;
+    t.stream = stream;
+    t.mark = mark;
+    return mark ? cudaEventRecord(mark, stream) : cudaSuccess;
+}
+
+void CooperativeTurn::leave() {
+    if (!number_) return;
+    Turns& t = turns_of(device_);
+    std::lock_guard<std::mutex> lock(t.mutex);
+    if (t.last == number_) t.busy = false;
+    number_ = 0;
 }
 
 cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
-                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, cudaStream_t stream) {
+                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, CooperativeTurn& turn,
+                                cudaEvent_t mark, cudaStream_t stream) {
     const FusedShape f = plan_coulomb(p, device_sms());
     if (!f.ept) return cudaErrorInvalidValue;
     FusedArgs a = f.a;
@@ -870,14 +904,17 @@ cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, 
     held.next += tags;
     a.err = err;
     a.wait_ns = wait_ns;
-    const bool more = long_sums(a);
-    switch (f.ept) {
-        case 1: return more ? launch_fused<1, true>(a, f.smem, stream) : launch_fused<1, false>(a, f.smem, stream);
-        case 2: return more ? launch_fused<2, true>(a, f.smem, stream) : launch_fused<2, false>(a, f.smem, stream);
-        case 3: return more ? launch_fused<3, true>(a, f.smem, stream) : launch_fused<3, false>(a, f.smem, stream);
-        case 4: return more ? launch_fused<4, true>(a, f.smem, stream) : launch_fused<4, false>(a, f.smem, stream);
-        default: return cudaErrorInvalidValue;
-    }
+    auto launch = [&] {
+        const bool more = long_sums(a);
+        switch (f.ept) {
+            case 1: return more ? launch_fused<1, true>(a, f.smem, stream) : launch_fused<1, false>(a, f.smem, stream);
+            case 2: return more ? launch_fused<2, true>(a, f.smem, stream) : launch_fused<2, false>(a, f.smem, stream);
+            case 3: return more ? launch_fused<3, true>(a, f.smem, stream) : launch_fused<3, false>(a, f.smem, stream);
+            case 4: return more ? launch_fused<4, true>(a, f.smem, stream) : launch_fused<4, false>(a, f.smem, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    };
+    return a.ge * a.gq > kCluster ? turn.enter(stream, mark, launch) : launch();
 }
 
 }  // namespace hf

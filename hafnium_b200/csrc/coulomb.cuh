@@ -24,15 +24,45 @@ struct PacketSpace {
     uint32_t next = 0;
 };
 
+// The turn of a cooperative grid on a device. Two such grids in flight could each hold SMs
+// that the other waits for, so a grid's stream first waits for the grid launched before
+// it; the host waits for neither. Under a lock held until a build had ended, a build also
+// waited for whatever another caller's stream still had to do, and eight threads' builds
+// took 44 us each at (H2O)4 and 75 at (H2O)8; now 34 and 53, in two passes 34 and 58.
+// Left, at the latest by the destructor, when the stream has been waited for.
+class CooperativeTurn {
+   public:
+    explicit CooperativeTurn(int device) : device_(device) {}
+    ~CooperativeTurn() { leave(); }
+    CooperativeTurn(const CooperativeTurn&) = delete;
+    CooperativeTurn& operator=(const CooperativeTurn&) = delete;
+    // Runs launch() in turn on `stream`. The next turn's stream waits for all work that is
+    // on this one by then, or, with an event, for `mark`, recorded right after the launch.
+    template <class Launch>
+    cudaError_t enter(cudaStream_t stream, cudaEvent_t mark, Launch launch) {
+        std::unique_lock<std::mutex> lock(mutex());
+        cudaError_t e = follow(stream);
+        if (e == cudaSuccess) e = launch();
+        if (e == cudaSuccess) e = take(stream, mark);
+        return e;
+    }
+    void leave();
+
+   private:
+    std::mutex& mutex();
+    cudaError_t follow(cudaStream_t stream);
+    cudaError_t take(cudaStream_t stream, cudaEvent_t mark);
+    int device_;
+    uint64_t number_ = 0;  // 0: not entered
+};
+
 // J = scale * sum_q (B_q . D) B_q, J full n x n. The grid's CTAs wait on one another,
 // bounded by wait_ns; past it *err (device-visible, 0 before) becomes 1 and J is
-// undefined (stall: a self-test in which one CTA's first packets are not sent). A small grid is one thread-block cluster; a larger one is cooperative
-// (coulomb_fused_cooperative): hold cooperative_mutex(device) from its launch to its
-// completion, since two such grids in flight could each hold SMs that the other waits for.
-bool coulomb_fused_cooperative(const JkPlan& p);
+// undefined (stall: a self-test in which the CTAs' packets carry tags that none waits
+// for). A small grid is one thread-block cluster; a larger one is cooperative and takes
+// its turn (mark: CooperativeTurn::enter).
 cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
-                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, cudaStream_t stream);
-
-std::mutex& cooperative_mutex(int device);
+                                PacketSpace& held, int* err, uint64_t wait_ns, int stall, CooperativeTurn& turn,
+                                cudaEvent_t mark, cudaStream_t stream);
 
 }  // namespace hf

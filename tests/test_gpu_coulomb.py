@@ -136,6 +136,63 @@ def test_a_wait_that_runs_out_costs_time_only(n, n_aux):
     assert torch.equal(inplace, before)
 
 
+def test_builds_of_several_contexts_at_once():
+    """Threads that build J of their own contexts (grids of every kind) get what one thread gets."""
+    import threading
+
+    import torch
+
+    sizes = [(24, 113), (48, 226), (192, 64), (288, 150), (520, 131), (777, 70)]
+    builders = [hydrogens(*size) for size in sizes]
+    densities, expected, wrong = [], [], []
+    for (n, _), two_body in zip(sizes, builders):
+        c = torch.randn((n, 5), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+        densities.append(c @ c.T)
+        expected.append(two_body.coulomb(densities[-1]))
+    torch.cuda.synchronize()
+
+    def work(i):
+        for _ in range(100):
+            if not torch.equal(builders[i].coulomb(densities[i]), expected[i]):
+                wrong.append(sizes[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong
+
+
+def test_a_build_does_not_wait_for_what_others_have_queued():
+    """J on a stream that still has other work is waited for by its caller alone."""
+    import threading
+    import time
+
+    import torch
+
+    busy, free = hydrogens(192, 64), hydrogens(288, 150)
+    stream = torch.cuda.Stream()
+    d = [torch.eye(t.n_ao, dtype=torch.float64, device="cuda") for t in (busy, free)]
+    out = [torch.empty_like(x) for x in d]
+    for t, x, y in zip((busy, free), d, out):
+        t.context.coulomb_device(x, y)
+    busy.context.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(2_000_000_000)  # about a second
+    thread = threading.Thread(target=busy.context.coulomb_device, args=(d[0], out[0]))
+    start = time.perf_counter()
+    thread.start()
+    time.sleep(0.1)
+    for _ in range(10):
+        free.context.coulomb_device(d[1], out[1])
+    took = time.perf_counter() - start
+    thread.join()
+    waited = time.perf_counter() - start
+    busy.context.set_stream(None)
+    assert waited > 0.5 and took < 0.5 * waited, (took, waited)
+
+
 def test_the_first_coulomb_builds_of_a_process():
     """The packets between CTAs are told by their tags from what the memory held before: a fresh process,
     whose tags start anew in memory that the build's integer lists have just used."""
