@@ -501,10 +501,12 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long ke
 }
 
 constexpr int kPivotThreads = 1024;
-constexpr int kPivotRows = 22;  // rows per thread (n <= 22528)
+constexpr int kPivotRows = 22;  // rows per thread that the shared diagonal has room for (n <= 22528)
 
 // One panel of up to `width` pivots of W (D itself for the first). Shared: d[n],
-// Lp[n][pitch] when it fits (else Lp is the global copy).
+// Lp[n][pitch] when it fits (else Lp is the global copy). WIDE, for larger n: the
+// diagonal and the used flags stay in global memory, keys have room for 2^20 rows.
+template <bool WIDE>
 __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __restrict__ W, int n, double tol, int maxr,
                                                             double* __restrict__ Lc, double* __restrict__ Lg,
                                                             int width, int pitch, int in_smem,
@@ -513,8 +515,10 @@ __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __rest
     extern __shared__ double psm[];
     __shared__ unsigned long long keys[2][32];
     __shared__ int s_bad;
-    double* d = psm;
-    double* Lp = in_smem ? psm + n : Lg;
+    constexpr int kBits = WIDE ? 20 : 16;  // of a key: the index
+    constexpr unsigned long long kIndex = (1ull << kBits) - 1;
+    double* d = WIDE ? dg : psm;
+    double* Lp = !WIDE && in_smem ? psm + n : Lg;
     const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5, warps = T >> 5;
     if (!first && st->stop) {
         if (tid == 0) {
@@ -524,12 +528,17 @@ __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __rest
         return;
     }
     unsigned mine = 0;  // bit m: row tid + m T has been a pivot
+    auto taken = [&](int i, int m) { return WIDE ? used[i] != 0 : (mine >> m & 1) != 0; };
     double top = 0.0;
     for (int i = tid, m = 0; i < n; i += T, ++m) {
         const double v = first ? W[(int64_t)i * n + i] : dg[i];
         d[i] = v;
-        if (first) top = fmax(top, fabs(v));
-        else if (used[i]) mine |= 1u << m;
+        if (first) {
+            top = fmax(top, fabs(v));
+            if (WIDE) used[i] = 0;
+        } else if (!WIDE && used[i]) {
+            mine |= 1u << m;
+        }
     }
     if (tid == 0) s_bad = 0;
     double dmax0;
@@ -547,19 +556,19 @@ __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __rest
     const int b = min(width, maxr - k0);
     int j = 0;
     for (; j < b; ++j) {
-        // the largest remaining diagonal entry, the lowest index among those equal to 2^-36 of it
+        // the largest remaining diagonal entry, the lowest index among those equal to 2^-36 (2^-32) of it
         unsigned long long key = 0;
         for (int i = tid, m = 0; i < n; i += T, ++m)
-            if (!(mine >> m & 1) && d[i] > 0.0) {
+            if (!taken(i, m) && d[i] > 0.0) {
                 const unsigned long long k =
-                    ((unsigned long long)__double_as_longlong(d[i]) & ~0xffffull) | (unsigned long long)(0xffff - i);
+                    ((unsigned long long)__double_as_longlong(d[i]) & ~kIndex) | (kIndex - (unsigned long long)i);
                 key = k > key ? k : key;
             }
         key = warp_max_key(key);
         if (lane == 0) keys[j & 1][warp] = key;
         __syncthreads();
         key = warp_max_key(lane < warps ? keys[j & 1][lane] : 0ull);
-        const int p = key ? 0xffff - (int)(key & 0xffff) : 0;
+        const int p = key ? (int)(kIndex - (key & kIndex)) : 0;
         const double best = key ? d[p] : 0.0;
         if (!(best > tol * dmax0)) break;
         const double piv = sqrt(best), inv = 1.0 / piv;
@@ -571,8 +580,9 @@ __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __rest
             double l = 0.0;
             if (i == p) {
                 l = piv;
-                mine |= 1u << m;
-            } else if (!(mine >> m & 1)) {
+                if (WIDE) used[i] = 1;
+                else mine |= 1u << m;
+            } else if (!taken(i, m)) {
                 const double wi = w[i];
                 const double* li = Lp + (int64_t)i * pitch;
                 double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
@@ -597,9 +607,11 @@ __global__ void __launch_bounds__(kPivotThreads) k_pc_panel(const double* __rest
     const bool stop = j < b || k0 + j >= maxr;
     int bad = 0;
     for (int i = tid, m = 0; i < n; i += T, ++m) {
-        const bool u = mine >> m & 1;
-        dg[i] = d[i];
-        used[i] = u;
+        const bool u = taken(i, m);
+        if (!WIDE) {
+            dg[i] = d[i];
+            used[i] = u;
+        }
         // indefinite if a remaining diagonal entry is clearly negative
         if (stop && !u && d[i] < -1e3 * tol * dmax0) bad = 1;
     }
@@ -841,6 +853,11 @@ namespace {
 // Pivots per panel and the pitch of its rows in shared memory (odd: rows of
 // consecutive threads in different banks); in_smem 0: rows in global memory.
 void pivot_panel(int n, int& width, int& pitch, int& in_smem) {
+    if (n > kPivotThreads * kPivotRows) {
+        width = pitch = 32;
+        in_smem = 0;
+        return;
+    }
     const int room = (int)((kPivotSmem - sizeof(double) * (size_t)n) / (sizeof(double) * (size_t)n));
     in_smem = room >= 9;
     pitch = in_smem ? std::min((room & 1) ? room : room - 1, n | 1) : 32;
@@ -859,7 +876,7 @@ size_t pivoted_cholesky_work_doubles(int n) {
 
 cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, double* work,
                                      int64_t* rank, int* indefinite, cudaStream_t stream, void* mapped) {
-    if (n < 1 || maxr < 1 || n > kPivotThreads * kPivotRows) return cudaErrorInvalidValue;
+    if (n < 1 || maxr < 1 || n > 1 << 20) return cudaErrorInvalidValue;
     cudaError_t e = jk_configure();
     if (e != cudaSuccess) return e;
     int width, pitch, in_smem;
@@ -869,7 +886,8 @@ cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int max
     double* d = Lg + (size_t)n * std::max(width, pitch);
     unsigned char* used = reinterpret_cast<unsigned char*>(d + n);
     PivotState* st = reinterpret_cast<PivotState*>(d + n + (n + 7) / 8);
-    const size_t smem = sizeof(double) * ((size_t)n + (in_smem ? (size_t)n * pitch : 0));
+    const bool wide = n > kPivotThreads * kPivotRows;
+    const size_t smem = wide ? 0 : sizeof(double) * ((size_t)n + (in_smem ? (size_t)n * pitch : 0));
     const int threads = std::min(kPivotThreads, std::max(128, (n + 31) / 32 * 32));
     const int panels = (maxr + width - 1) / width;
     // A density's rank is its occupied orbitals, about a fifth of n: panels for 0.3 n are queued
@@ -900,9 +918,9 @@ cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int max
                 e = dgemm_nt(g, 1, stream);
                 if (e != cudaSuccess) return e;
             }
-            k_pc_panel<<<1, threads, smem, stream>>>(queued == 0 ? D : W, n, tol, maxr, Lc, Lg, width, pitch, in_smem, d,
-                                                     used, queued == 0 ? 1 : 0, st,
-                                                     queued + 1 == until ? static_cast<PivotState*>(mapped) : nullptr);
+            (wide ? k_pc_panel<true> : k_pc_panel<false>)<<<1, threads, smem, stream>>>(
+                queued == 0 ? D : W, n, tol, maxr, Lc, Lg, width, pitch, in_smem, d, used, queued == 0 ? 1 : 0, st,
+                queued + 1 == until ? static_cast<PivotState*>(mapped) : nullptr);
         }
         e = mapped ? cudaSuccess : cudaMemcpyAsync(&host, st, sizeof(host), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -951,7 +969,7 @@ cudaError_t jk_configure() {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_pivoted_cholesky, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_pc_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmem);
+    e = cudaFuncSetAttribute(k_pc_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPivotSmem);
     if (e != cudaSuccess) return e;
     g_jk_configured[dev] = true;
     return dgemm_configure();

@@ -71,7 +71,7 @@ cudaError_t pivoted_cholesky(const double* D, int64_t strideD, int n, double tol
 // product once per panel of pivots; the pivots and the factor are those of
 // pivoted_cholesky up to rounding. Waits for the stream: *rank and *indefinite are
 // the host's, read from `mapped` (kPivotMapped bytes of page-locked host memory that
-// the kernel writes) or, when that is null, by a copy. n <= 22528.
+// the kernel writes) or, when that is null, by a copy. n <= 2^20.
 constexpr size_t kPivotMapped = 32;
 size_t pivoted_cholesky_work_doubles(int n);
 cudaError_t pivoted_cholesky_blocked(const double* D, int n, double tol, int maxr, double* Lc, double* work,

@@ -5,10 +5,9 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from hafnium_b200.basis import ShellTable
-from hafnium_b200.jk import B200DensityFittedCoulombExchange
+from hafnium_b200 import _lib
 from hafnium_b200.molecule import water_cluster
-from tests.test_gpu_coulomb import hydrogens
+from tests.test_gpu_coulomb import hydrogen_tables, hydrogens
 
 pytestmark = pytest.mark.gpu
 EPS = 2.3e-16
@@ -53,6 +52,24 @@ def test_density_factor_across_panels(n, rank):
     # remainder it stops at is 1e-14 of the largest diagonal element
     bound = ((rank + 2) * EPS + 1e-14) * float(d.diagonal().max()) * 4
     assert float((f @ f.T - d).abs().max()) < bound
+
+
+# the narrowest panels with their rows in shared memory and the first without, the largest n whose diagonal
+# is there too and the first without; several panels each
+@pytest.mark.parametrize("n,rank", [(2560, 33), (2560, 70), (2561, 33), (2561, 70), (22528, 40), (22529, 40)])
+def test_density_factor_of_large_matrices(n, rank):
+    import torch
+
+    context = _lib.Context()
+    context.upload(hydrogen_tables(n, 1)[0])
+    gen = torch.Generator().manual_seed(n + rank)
+    c = torch.randn((n, rank), dtype=torch.float64, generator=gen).cuda() / np.sqrt(n)
+    d = c @ c.T
+    f = context.density_factor_device(d, rank + 30)
+    assert rank <= f.shape[1] <= rank + 30
+    # as above
+    bound = ((rank + 2) * EPS + 1e-14) * float(d.diagonal().max()) * 4
+    assert max(float((part @ f.T - rows).abs().max()) for part, rows in zip(f.split(2048), d.split(2048))) < bound
 
 
 # blocks of 64: one, a ragged one, several, with and without a remainder
