@@ -952,7 +952,16 @@ const char* hf_batch_last_error(const hf_batch* b) { return b ? b->err.c_str() :
 
 int hf_batch_set_stream(hf_batch* b, void* stream) {
     if (!b) return HF_ERR_ARG;
-    b->stream = stream ? (cudaStream_t)stream : b->own;
+    cudaStream_t next = stream ? (cudaStream_t)stream : b->own;
+    if (next != b->stream) {
+        // as hf_set_stream: what an error has left on the old stream finishes before the switch
+        cudaSetDevice(b->device);
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(b->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+            cudaStreamSynchronize(b->stream);
+        cudaGetLastError();
+    }
+    b->stream = next;
     return HF_OK;
 }
 
@@ -1026,7 +1035,7 @@ int check_options(hf_batch* b, const hf_batch_options& o) {
 
 // Resets the per-run state (a load leaves it reset; a second run starts again
 // from the loaded guess only after another load).
-int run_group(hf_batch* const* batches, int nb, const hf_batch_options& o) {
+int queue_group(hf_batch* const* batches, int nb, const hf_batch_options& o) {
     hf_batch* b = batches[0];
     cudaStream_t s = b->stream;
     const int max_bodies = o.max_iterations + 2;
@@ -1171,6 +1180,17 @@ int run_group(hf_batch* const* batches, int nb, const hf_batch_options& o) {
     HB_CU(cudaStreamSynchronize(s));
     for (int i = 0; i < nb; ++i) batches[i]->loaded = false;
     return HF_OK;
+}
+
+// All batches run on the first one's stream, and a batch's blocks go back to the pool in
+// the order of its own: after an error, too, nothing of the run is left behind there.
+int run_group(hf_batch* const* batches, int nb, const hf_batch_options& o) {
+    const int status = queue_group(batches, nb, o);
+    if (status != HF_OK) {
+        cudaStreamSynchronize(batches[0]->stream);
+        cudaGetLastError();
+    }
+    return status;
 }
 
 }  // namespace
