@@ -194,8 +194,7 @@ def test_a_build_does_not_wait_for_what_others_have_queued():
 
 
 def test_the_first_coulomb_builds_of_a_process():
-    """The packets between CTAs are told by their tags from what the memory held before: a fresh process,
-    whose tags start anew in memory that the build's integer lists have just used."""
+    """The first J of a context, in memory that the build's integer lists have just used, equals the second."""
     import subprocess
     import sys
 

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from hafnium_b200 import _lib
+from hafnium_b200.errors import InputError
 from hafnium_b200.molecule import water_cluster
 from tests.test_gpu_coulomb import hydrogen_tables, hydrogens
 
@@ -34,6 +35,71 @@ def test_exchange_of_every_column_tile(columns, signed):
     size = torch.einsum("qui,qvi->uv", ax if w is None else ax * w.abs(), ax)
     got = two_body.exchange_factored(c, w)
     assert float(((got - expected).abs() / ((2 * n + n_aux * columns) * EPS * size)).max()) < 1.0
+
+
+# X's rows in several chunks (4 GB in FP64, 2 GB in split BF16, half as many rows with a signed factor): K is
+# then added up chunk by chunk
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("precision", [_lib.PREC_FP64, _lib.PREC_BF16X3])
+def test_exchange_in_several_chunks_of_rows(signed, precision):
+    import torch
+
+    n, n_aux, columns = 1030, 600, 1000
+    two_body = hydrogens(n, n_aux)
+    gen = torch.Generator().manual_seed(columns)
+    c = torch.randn((n, columns), dtype=torch.float64, generator=gen).cuda()
+    w = torch.randn(columns, dtype=torch.float64, generator=gen).cuda() if signed else None
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    b = two_body.orbital_tensor(eye, eye)
+    expected, size = torch.zeros_like(eye), torch.zeros_like(eye)
+    for q in range(0, n_aux, 50):
+        x, ax = b[q:q + 50] @ c, b[q:q + 50].abs() @ c.abs()
+        expected += torch.einsum("qui,qvi->uv", x if w is None else x * w, x)
+        size += torch.einsum("qui,qvi->uv", ax if w is None else ax * w.abs(), ax)
+    for _ in range(2):
+        got = two_body.exchange_factored(c, w, precision)
+        error = (got - expected).abs()
+        if precision == _lib.PREC_FP64:  # two sums of n, then n_aux columns products
+            assert float((error / ((2 * n + n_aux * columns) * EPS * size)).max()) < 1.0
+        else:
+            # 16 bits of each factor, and each addition of 16 products to a 32-bit sum truncates by up to 2^-23: a
+            # chunk's 450 rows of 1000 columns in three products, split twelve ways, are 7000 additions, 8e-4; a
+            # signed sum against its parts
+            scale = expected if w is None else two_body.exchange_factored(c, w.abs())
+            assert float(error.max()) <= 1e-3 * float(scale.abs().max())
+        assert torch.equal(got, got.T)
+
+
+def test_a_context_without_a_word_of_mapped_memory():
+    """The page of words that kernels write for the host has 1024 of them; later contexts copy, and their J is
+    built in two passes."""
+    import torch
+
+    n, n_aux = 129, 300
+    c = torch.randn((n, 20), dtype=torch.float64, generator=torch.Generator().manual_seed(n)).cuda()
+    d = c @ c.T
+    contexts = [_lib.Context() for _ in range(1026)]
+    results = []
+    for context in (contexts[0], contexts[-1]):
+        context.upload(*hydrogen_tables(n, n_aux))
+        context.build()
+        j, k, k16 = torch.empty_like(d), torch.empty_like(d), torch.empty_like(d)
+        before = context.stats()["kernel_launches"]
+        context.coulomb_device(d, j)
+        launches = context.stats()["kernel_launches"] - before
+        context.exchange_device(d, k)
+        context.exchange_device(d, k16, _lib.PREC_BF16X3)
+        f = context.density_factor_device(d, n)
+        results.append((launches, j, k, k16, f))
+        with pytest.raises(InputError, match="semidefinite"):
+            context.density_factor_device(-d, n)
+    (first, j0, *others), (last, j1, *same) = results
+    assert (first, last) == (1, 4)
+    assert float((j0 - j1).abs().max()) < 2.3e-16 * (n * n + n_aux) * float(j0.abs().max())
+    for x, y in zip(others, same):
+        assert torch.equal(x, y)
+    for context in contexts:
+        context.close()
 
 
 # one panel and several, rows of L in shared memory, ranks that end inside and at the end of a panel
