@@ -32,12 +32,13 @@
 //     (polling the host's flag took up to 100 us).
 //
 // Measured on one B200 (kernels of one J with the timing events, two-pass ->
-// one-pass): (H2O)8 153 -> 64 us, (H2O)12 240 -> 139, (H2O)16 457 -> 282,
-// (H2O)32 2741 -> 2100 (8.55 GB: 4.1 TB/s; without the exchange of c it runs in
-// 1600, so what is left is the latency of two hops), (H2O)44 7120 -> 5670. Past
-// four pieces per thread (n about 1100) registers spill and the rows that tensor
-// memory holds no longer cover the exchange: six pieces measured 7.9 ms at n =
-// 1152 without the exchange and three times that with it, against 8.7 in two passes.
+// one-pass): (H2O)8 153 -> 61 us, (H2O)12 240 -> 134, (H2O)16 457 -> 280,
+// (H2O)32 2741 -> 1870 (8.55 GB: 4.6 TB/s; without the exchange of c it runs in
+// 1600, so what is left is the latency of two hops and 130 for the long sums),
+// (H2O)44 7120 -> 5120. Past four pieces per thread (n about 1100) registers spill
+// and the rows that tensor memory holds no longer cover the exchange: six pieces
+// measured 7.9 ms at n = 1152 without the exchange and three times that with it,
+// against 8.7 in two passes.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -745,7 +746,11 @@ int64_t upper_pieces(int64_t n, int nt) {
 bool long_sums(const FusedArgs& a) { return a.blocks >= a.flush; }
 
 constexpr int kMaxPieces = 4;         // pieces of a row per thread
-constexpr int64_t kSmallPieces = 20000;  // up to here one cluster of 8 CTAs holds everything (one water: 23.5 us, 27 spread out)
+// Up to this many pieces (rows times pieces of a row) one cluster of 8 CTAs holds everything; past it
+// the rows are spread out over groups. Whole calls, cluster against spread out: 1800 pieces (n = 7) 39.0
+// and 40.8 us, 12700 (n = 14) 43.6 and 44.4, 17600 (one water, n = 24) 41.9 and 42.6, 44000 (n = 21) 46.8
+// and 44.7, 95000 (n = 28) 49.8 and 44.6.
+constexpr int64_t kSmallPieces = 20000;
 
 // How the work is laid out; ept == 0 when the fused form does not apply.
 struct FusedShape {

@@ -478,12 +478,13 @@ __global__ void __launch_bounds__(1024) k_pivoted_cholesky(const double* __restr
 // once per panel.
 //
 // A panel is one CTA's chain of pivots, so a pivot's latency is what counts. The
-// panel's rows of L sit in shared memory (as many pivots per panel as fit: all of
-// them up to n = 160, 94 at n = 288, 16 at n = 1536), the pivot is found with one
-// barrier (64-bit keys of value and index, reduced by two 32-bit warp reductions
-// each), the pivot's row of W is on its way while the corrections are summed, and
-// no division is in the chain. Per pivot about 0.6 us, where the rows of L in
-// global memory and two shuffled reductions took 4 (n = 48) to 20 us (n = 1536).
+// panel's rows of L sit in shared memory (as many pivots per panel as fit: 158 at
+// n = 160, 86 at n = 288, 14 at n = 1536, 8 at n = 2560; past that 32, with the rows
+// in global memory), the pivot is found with one barrier (64-bit keys of value and
+// index, reduced by two 32-bit warp reductions each), the pivot's row of W is on its
+// way while the corrections are summed, and no division is in the chain. Per pivot
+// about 0.6 us, where the rows of L in global memory and two shuffled reductions took
+// 4 (n = 48) to 20 us (n = 1536).
 struct PivotState {
     double dmax0;  // the largest initial diagonal entry
     int k;         // pivots taken

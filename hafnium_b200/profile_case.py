@@ -119,7 +119,8 @@ def main() -> None:
     n, naux, o = ham.n_ao, two_body.n_aux, int(kfac.shape[1])
     out["exchange_fp64_tflops"] = 4.0 * naux * n * n * o / (out["exchange_fp64_ms"] / 1e3) / 1e12
     out["exchange_bf16_exec_tflops"] = 3 * 4.0 * naux * n * n * o / (out["exchange_bf16_ms"] / 1e3) / 1e12
-    out["coulomb_gbs"] = 2.0 * two_body.stats()["b_bytes"] / (out["coulomb_ms"] / 1e3) / 1e9
+    # B's upper triangle once, whatever the build reads (past about 1100 functions J takes two passes)
+    out["coulomb_gbs"] = 4.0 * naux * n * (n + 1) / (out["coulomb_ms"] / 1e3) / 1e9
     if args.gradient:
         from hafnium_b200.gradient import gradient_from_state
 
