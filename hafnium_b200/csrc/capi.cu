@@ -1355,17 +1355,22 @@ static int coulomb_run(hf_ctx* ctx, const JkPlan& p, const CoulombRun& run, cons
         // what a caller has queued on a stream of its own may wait for another context's build: it must not
         // stand between this build's turn and its grid, nor may what is queued behind the grid
         const bool own = ctx->stream == ctx->own;
-        if (!own) HF_CU(cudaStreamSynchronize(ctx->stream));
+        if (!own && coulomb_fused_cooperative(p)) HF_CU(cudaStreamSynchronize(ctx->stream));
         CooperativeTurn turn(ctx->device);
         const int stall = ctx->stall_coulomb;
         ctx->stall_coulomb = 0;
-        HF_CU(coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, kCoulombWaitNs, stall, turn,
-                                  own ? nullptr : ctx->ev1, ctx->stream));
-        ++ctx->stats.kernel_launches;
-        if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        const int s = check_async(ctx, what);
-        if (s != HF_OK || *(volatile int*)ctx->h_flag == 0) return s;
-        *(volatile int*)ctx->h_flag = 0;
+        const cudaError_t e = coulomb_build_fused(p, D, 1.0, J, work, held, ctx->h_flag, kCoulombWaitNs, stall, turn,
+                                                  own ? nullptr : ctx->ev1, ctx->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            cudaGetLastError();  // the process may use fewer SMs than the device has: two passes
+        } else {
+            HF_CU(e);
+            ++ctx->stats.kernel_launches;
+            if (host_out) HF_CU(cudaMemcpyAsync(host_out, J, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            const int s = check_async(ctx, what);
+            if (s != HF_OK || *(volatile int*)ctx->h_flag == 0) return s;
+            *(volatile int*)ctx->h_flag = 0;
+        }
     }
     held.next = 0;
     HF_CU(coulomb_build(p, D, J, work, ctx->stream));

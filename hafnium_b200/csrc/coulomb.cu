@@ -834,6 +834,11 @@ size_t coulomb_fused_work_doubles(const JkPlan& p) {
     return (tagged_bytes(f.a) + jpart_bytes(f.a) + jsum_bytes(f.a)) / 8 + 2;
 }
 
+bool coulomb_fused_cooperative(const JkPlan& p) {
+    const FusedShape f = plan_coulomb(p, device_sms());
+    return f.ept && f.a.ge * f.a.gq > kCluster;
+}
+
 namespace {
 struct Turns {
     std::mutex mutex;

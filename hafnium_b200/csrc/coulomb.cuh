@@ -61,6 +61,7 @@ class CooperativeTurn {
 // undefined (stall: a self-test in which the CTAs' packets carry tags that none waits
 // for). A small grid is one thread-block cluster; a larger one is cooperative and takes
 // its turn (mark: CooperativeTurn::enter).
+bool coulomb_fused_cooperative(const JkPlan& p);
 cudaError_t coulomb_build_fused(const JkPlan& p, const double* D, double scale, double* J, double* work,
                                 PacketSpace& held, int* err, uint64_t wait_ns, int stall, CooperativeTurn& turn,
                                 cudaEvent_t mark, cudaStream_t stream);

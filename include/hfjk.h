@@ -151,7 +151,11 @@ int hf_set_fitted_rows(hf_ctx* ctx, int64_t row0, int64_t row1);
 
 int hf_dims(const hf_ctx* ctx, int64_t* n_ao, int64_t* n_aux);
 
-/* J[u][v] = sum_wx (uv|wx) D[w][x] (coulomb_exchange.py:176-182). */
+/* J[u][v] = sum_wx (uv|wx) D[w][x] (coulomb_exchange.py:176-182), in one pass over
+ * the fitted tensor up to about 1100 functions and in two beyond. Builds of
+ * several contexts on one device may run at once; the one-pass grids of one
+ * device run one after the other on the GPU, without the callers waiting for one
+ * another. J may be D's array. */
 int hf_coulomb(hf_ctx* ctx, const double* density, double* coulomb, int on_device);
 
 /* The J build of hf_coulomb without any device allocation, for callers that
