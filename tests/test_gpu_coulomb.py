@@ -68,7 +68,8 @@ def pairwise(x):
     return x[0]
 
 
-@pytest.mark.parametrize("n,n_aux", [(450, 1200), (800, 2000)])
+# rows side by side in one cluster, several groups, one group
+@pytest.mark.parametrize("n,n_aux", [(5, 1400), (450, 1200), (800, 2000)])
 def test_the_running_sums_of_j_are_short(n, n_aux):
     """Rounding errors of a running sum add up like its partial sums' squares; J errs no more than sums of 88
     rows, added up, do (one sum over all rows errs five times as much)."""
