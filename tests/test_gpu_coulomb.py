@@ -91,7 +91,9 @@ def test_the_running_sums_of_j_are_short(n, n_aux):
     # each rounding errs by at most 2^-53 of the partial sum, 1 / sqrt(3) of that in the mean square; twice
     # that for the charges' own errors, which are of the size of one more addition
     expected = 2 * 2.0**-53 / 3**0.5 * float(squares.sum().sqrt())
-    assert float((two_body.coulomb(d) - pairwise(totals)).norm()) < expected
+    got = two_body.coulomb(d)
+    assert float((got - pairwise(totals)).norm()) < expected
+    assert torch.equal(two_body.coulomb(d), got)  # sums in a fixed order
 
 
 # one cluster, groups that meet only in J, collectors by lanes, by warps and through owners, few and
